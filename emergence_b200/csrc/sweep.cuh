@@ -29,6 +29,7 @@
 // and c+1.
 #pragma once
 #include "physics.cuh"
+#include "quotient.cuh"
 #include "tma.cuh"
 #include <stdint.h>
 
@@ -107,6 +108,7 @@ struct SweepParams {
     // high-order flux was kept); read back by the discrete adjoint
     double* theta_rec;
     int64_t nface;  // elements of `face` (bounds-check build)
+    double cfl_rdx[3];  // 1/cfl_dx
 };
 
 // index check of the bounds-check build: true when 0 <= i < n; otherwise the
@@ -289,6 +291,74 @@ struct Sweep {
         hllc(e, wl, wr, un, f);
     }
 
+    // The same values from the branch-free quotients and square roots of
+    // quotient.cuh; false (f not set) when an operand leaves their ranges or an
+    // interpolated state is inadmissible.
+    __device__ static __forceinline__ bool midpoint_rn(const Eos<double>& e, const RecipRn& rg,
+                                                       const double* __restrict__ Wd, int m, int l, double* f) {
+        constexpr int un = 1 + D;
+        constexpr int t1 = 1 + (D + 1) % 3, t2 = 1 + (D + 2) % 3;
+        const int j = m + 2;
+        bool bad = false;
+        const double rho = 0.5 * (Wd[at<STRW>(j, 0, l)] + Wd[at<STRW>(j + 1, 0, l)]);
+        const double p4 = 0.5 * (Wd[at<STRW>(j, 4, l)] + Wd[at<STRW>(j + 1, 4, l)]);
+        const RecipRn ir = den_rn(rho, bad);
+        const double c = sound_speed_rn(e, p4, ir.y, bad);
+        // ρ/(2c) = ½·(ρ/c) and 1/(2c·c) = ½·(1/(c·c)) exactly
+        const double l4un = 0.5 * div_rn(rho, den_rn(c, bad), bad);
+        const double l0un = -l4un;
+        const double icc = den_rn(c * c, bad).y;
+        const double l04 = 0.5 * icc;
+        const double l14 = -icc;
+        const double run4 = quot_rn(c, ir);
+        const double run0 = -run4;
+        const double r40 = c * c;
+        double cl[5], cr[5];
+#pragma unroll
+        for (int a = 0; a < 5; a++) {
+            double ch[6];
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                const int row = m + s;
+                switch (a) {
+                    case 0: ch[s] = l0un * Wd[at<STRW>(row, un, l)] + l04 * Wd[at<STRW>(row, 4, l)]; break;
+                    case 1: ch[s] = Wd[at<STRW>(row, 0, l)] + l14 * Wd[at<STRW>(row, 4, l)]; break;
+                    case 2: ch[s] = Wd[at<STRW>(row, t1, l)]; break;
+                    case 3: ch[s] = Wd[at<STRW>(row, t2, l)]; break;
+                    default: ch[s] = l4un * Wd[at<STRW>(row, un, l)] + l04 * Wd[at<STRW>(row, 4, l)];
+                }
+            }
+            weno5z_pair_rn(ch, cl[a], cr[a], bad);
+        }
+        double wl[5], wr[5];
+        wl[0] = (cl[0] + cl[1]) + cl[4];
+        wr[0] = (cr[0] + cr[1]) + cr[4];
+        wl[un] = run0 * cl[0] + run4 * cl[4];
+        wr[un] = run0 * cr[0] + run4 * cr[4];
+        wl[t1] = cl[2];
+        wr[t1] = cr[2];
+        wl[t2] = cl[3];
+        wr[t2] = cr[3];
+        wl[4] = r40 * cl[0] + r40 * cl[4];
+        wr[4] = r40 * cr[0] + r40 * cr[4];
+        const double vl = den_rn(wl[0], bad).y, vr = den_rn(wr[0], bad).y;
+        // an inadmissible state has no positive ρ, 1/ρ − b or p + p∞ and is refused
+        // by its sound speed (c² ≤ 0 or not finite) at the latest
+        hllc_rn(e, rg, wl, wr, vl, vr, un, f, bad);
+        return !bad;
+    }
+    // the same midpoint with the compiler's division, straight into the flux
+    // ring: only for operands outside the branch-free quotients' ranges
+    __device__ static __noinline__ bool midpoint_div(const Eos<double> e, const double* __restrict__ W, double* MF, int m,
+                                                     int l) {
+        double f[5];
+        bool fb;
+        midpoint<STRW>(e, W, m, l, f, fb);
+#pragma unroll
+        for (int k = 0; k < 5; k++) MF[atM(m, k, l)] = f[k];
+        return fb;
+    }
+
     // Mixed form of the midpoint flux: the characteristic projection, the
     // back-projection, the admissibility test and the HLLC flux in FP64 (its
     // wave-speed bounds from FP32 sound speeds, hllc_fs), with Newton-refined
@@ -430,6 +500,43 @@ struct Sweep {
         hllc_f(e, igm1, wl, wr, un, f);
     }
 
+    // maps and quotients of the plain form, redone with the compiler's
+    // division where an operand leaves the branch-free ranges
+    __device__ static __noinline__ double div_slow(double a, double b) { return a / b; }
+    __device__ static __forceinline__ double quot_plain(double a, const RecipRn& d, bool out) {
+        return out || num_out(a) ? div_slow(a, d.b) : quot_rn(a, d);
+    }
+    __device__ static __noinline__ double pressure_slow(const Eos<double> e, double r, double mx, double my, double mz,
+                                                        double en) {
+        const double u[5] = {r, mx, my, mz, en};
+        double w[5];
+        to_prim(e, u, w);
+        return w[4];
+    }
+    __device__ static __forceinline__ void to_prim_plain(const Eos<double>& e, const double* u, double* w) {
+        bool bad = false;
+        to_prim_rn(e, u, w, bad);
+        if (bad) {
+            w[1] = div_slow(u[1], u[0]);
+            w[2] = div_slow(u[2], u[0]);
+            w[3] = div_slow(u[3], u[0]);
+            w[4] = pressure_slow(e, u[0], u[1], u[2], u[3], u[4]);
+        }
+    }
+    __device__ static __noinline__ double sound_slow(const Eos<double> e, double rho, double p) { return sound_speed(e, rho, p); }
+    __device__ static __forceinline__ double sound_speed_plain(const Eos<double>& e, double rho, double p) {
+        bool bad = false;
+        const double c = sound_speed_rn(e, p, den_rn(rho, bad).y, bad);
+        return bad ? sound_slow(e, rho, p) : c;
+    }
+    __device__ static __noinline__ double rho_e_slow(const Eos<double> e, double rho, double p) { return e.rho_e(rho, p); }
+    __device__ static __forceinline__ void to_cons_plain(const Eos<double>& e, const RecipRn& rg, bool rg_out,
+                                                         const double* w, double* u) {
+        bool bad = rg_out;
+        to_cons_rn(e, rg, w, den_rn(w[0], bad).y, u, bad);
+        if (bad) u[4] = rho_e_slow(e, w[0], w[4]) + 0.5 * w[0] * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]);
+    }
+
     // KEEP-PE two-point flux with cached ρe (C/system.rs:317-334).
     __device__ static __forceinline__ void split_flux(const double* __restrict__ W, int ra, int rb, int l, double* f) {
         constexpr int un = 1 + D;
@@ -478,17 +585,17 @@ struct Sweep {
     // nothing over- or underflows. Whenever it holds, the reference's test
     // (to_prim: ein = E/ρ − ½|u|², p = (γ−1)·ein/(1/ρ); then ρ > 0, p > 0,
     // both finite, 1/ρ > 0) holds as well: the computed ein is within a few
-    // ulps of (2ρE − |ρu|²)/(2ρ²), far inside the margin. Where it does not
-    // hold, the reference's test runs as is, so the decision is always the
-    // reference's.
+    // ulps of (2ρE − |ρu|²)/(2ρ²), far inside the margin, as are the roundings
+    // of this test. Where it does not hold, the reference's test runs as is, so
+    // the decision is always the reference's. The bounds (2^±332) and the sign
+    // are tested on the high words, off the FP64 pipe.
     __device__ static __forceinline__ bool surely_admissible(const double* a) {
-        const double r = a[0], E = a[4];
-        if (!(r > 1e-100 && r < 1e100 && E > 1e-100 && E < 1e100 && fabs(a[1]) < 1e100 && fabs(a[2]) < 1e100 &&
-              fabs(a[3]) < 1e100))
-            return false;
-        const double m2 = a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
-        const double twore = 2.0 * r * E;
-        return twore - m2 > 1e-11 * (twore + m2);
+        const unsigned hr = hi_bits(a[0]), hE = hi_bits(a[4]);
+        const unsigned hm = max(hi_bits(a[1]) & 0x7fffffffu, max(hi_bits(a[2]) & 0x7fffffffu, hi_bits(a[3]) & 0x7fffffffu));
+        constexpr unsigned LO = (1023u - 332u) << 20, HI = (1023u + 332u) << 20;
+        const double m2 = fma(a[3], a[3], fma(a[2], a[2], a[1] * a[1]));
+        const double d = fma(2.0 - 2e-11, a[0] * a[4], -(1.0 + 1e-11) * m2);
+        return hr - LO < HI - LO && hE - LO < HI - LO && hm < HI && __double2hiint(d) > 0;
     }
 
     // one-sided admissibility of the limiter (C/scheme.rs:408-416), in f64;
@@ -661,7 +768,11 @@ struct Sweep {
         const bool lim_on = p.positivity && lam > 0.0;  // C/scheme.rs:278
         const double inv = 1.0 / dx;
         const bool ideal_gas = ed.b == 0.0 && ed.q == 0.0 && ed.p_inf == 0.0 && ed.gamma > 1.0 && ed.gamma < 100.0;
-        const double igm1 = FMAPS ? 1.0 / (ed.gamma - 1.0) : 0.0;  // fast maps: 1/(γ − 1)
+        const double igm1 = 1.0 / (ed.gamma - 1.0);
+        // correctly rounded reciprocals of the plain form's fixed divisors; one
+        // outside the branch-free range sends its quotients to the slow path
+        const RecipRn rg{ed.gamma - 1.0, igm1}, rdx{dx, inv}, r3{3.0, 1.0 / 3.0};
+        const bool rg_out = den_out(rg.b), dx_out = den_out(dx);
         __syncthreads();  // lane table
         const int Lmax = BATCH ? s_maxlen : Ls;
         const int nrounds = (Lmax + 5 + RM - 1) / RM;
@@ -734,7 +845,7 @@ struct Sweep {
                         if constexpr (FMAPS)
                             to_prim_f(ed, u, w);
                         else
-                            to_prim(ed, u, w);
+                            to_prim_plain(ed, u, w);
 #pragma unroll
                         for (int k = 0; k < 5; k++) W[at<STRW>(row, k, l)] = w[k];
                         if constexpr (MODE != MODE_WENO)
@@ -767,7 +878,7 @@ struct Sweep {
                         if constexpr (FMAPS)
                             to_prim_f(ed, u, w);
                         else
-                            to_prim(ed, u, w);
+                            to_prim_plain(ed, u, w);
 #pragma unroll
                         for (int k = 0; k < 5; k++) {
                             W[at<STRW>(row, k, l)] = w[k];
@@ -819,15 +930,19 @@ struct Sweep {
                     }
                     if (need) {
                         double f[5];
-                        bool fb;
+                        bool fb = false, done = true;
                         if constexpr (MIXED)
                             midpoint_mixed(ed, W, m, l, f, fb);
                         else if constexpr (FAST)
                             midpoint_fast(ed, igm1, W, m, l, f, fb);
                         else
-                            midpoint<STRW>(ed, W, m, l, f, fb);
+                            done = !rg_out && midpoint_rn(ed, rg, W, m, l, f);
+                        if (done) {
 #pragma unroll
-                        for (int k = 0; k < 5; k++) MF[atM(m, k, l)] = f[k];
+                            for (int k = 0; k < 5; k++) MF[atM(m, k, l)] = f[k];
+                        } else if constexpr (!FMAPS) {
+                            fb = midpoint_div(ed, W, MF, m, l);
+                        }
                         if (fb && (m < lane_len(l) || lane_tail(l))) atomicAdd(&s_fallback, chain_mult(m, 5));
                     }
                 }
@@ -890,14 +1005,14 @@ struct Sweep {
                             to_cons_f(ed, igm1, wi, ul);
                             to_cons_f(ed, igm1, wj, ur);
                         } else {
-                            to_cons(ed, wi, ul);
-                            to_cons(ed, wj, ur);
+                            to_cons_plain(ed, rg, rg_out, wi, ul);
+                            to_cons_plain(ed, rg, rg_out, wj, ur);
                         }
                         flux_wq(wi, ul, un, flp);
                         flux_wq(wj, ur, un, frp);
                         bool finite = true;
 #pragma unroll
-                        for (int k = 0; k < 5; k++) finite = finite && isfinite(fh[k]);
+                        for (int k = 0; k < 5; k++) finite = finite && (hi_bits(fh[k]) & 0x7ff00000u) != 0x7ff00000u;
                         if (!(finite && lim_ok(ed, fh, ul, flp, ur, frp, lam2_l, ideal_gas))) {
                             const double alpha = fmax(fabs(wi[un]) + sound_speed(ed, wi[0], wi[4]),
                                                       fabs(wj[un]) + sound_speed(ed, wj[0], wj[4]));
@@ -964,7 +1079,7 @@ struct Sweep {
                     for (int k = 0; k < 5; k++) {
                         // the block solver divides by dx (C/amr.rs:1263), the uniform one multiplies by 1/dx
                         const double df = F[atF(c + 1, k, l)] - F[atF(c, k, l)];
-                        const double x = AMR ? df / dx : df * inv_l;
+                        const double x = AMR ? quot_plain(df, rdx, dx_out) : df * inv_l;
                         const double prev = p.first ? 0.0 : p.rhs[k * p.ncell + g];
                         res[k] = prev - x;
                     }
@@ -982,7 +1097,7 @@ struct Sweep {
                             } else if (p.stage == 2) {
                                 v = 0.75 * o + 0.25 * (p.cur[k * p.ncell + g] + dt_l * res[k]);
                             } else {
-                                v = p.cur[k * p.ncell + g] / 3.0 + (2.0 / 3.0) * (o + dt_l * res[k]);
+                                v = quot_plain(p.cur[k * p.ncell + g], r3, false) + (2.0 / 3.0) * (o + dt_l * res[k]);
                             }
                             p.dest[k * p.ncell + g] = v;
                             un_[k] = v;
@@ -1000,12 +1115,14 @@ struct Sweep {
                                 for (int dd = 0; dd < 3; dd++)
                                     if (p.cfl_active[dd]) acc = acc + (fabs(w[1 + dd]) + cs) * rcp_f(p.cfl_dx[dd]);
                             } else {
-                                to_prim(ed, un_, w);
+                                to_prim_plain(ed, un_, w);
                                 if (!admissible(ed, w[0], w[4])) bad_state = 1;
-                                const double cs = sound_speed(ed, w[0], w[4]);
+                                const double cs = sound_speed_plain(ed, w[0], w[4]);
 #pragma unroll
                                 for (int dd = 0; dd < 3; dd++)
-                                    if (p.cfl_active[dd]) acc = acc + (fabs(w[1 + dd]) + cs) / p.cfl_dx[dd];
+                                    if (p.cfl_active[dd])
+                                        acc = acc + quot_plain(fabs(w[1 + dd]) + cs, RecipRn{p.cfl_dx[dd], p.cfl_rdx[dd]},
+                                                               den_out(p.cfl_dx[dd]));
                             }
                             rate_max = fmax(rate_max, acc);
                         }

@@ -658,6 +658,7 @@ int launch_axis(emg_uniform* h, int stage, int d, double* in, bool first, bool l
                 for (int k = 0; k < 3; k++) {
                     p.cfl_active[k] = h->active[k];
                     p.cfl_dx[k] = h->mesh.dx[k];
+                    p.cfl_rdx[k] = 1.0 / h->mesh.dx[k];
                 }
             }
         }
