@@ -391,8 +391,9 @@ struct emg_five {
         stream = nullptr;
     }
 
-    // launch shape per axis: P pencils per CTA along the lane axis, segments
-    // shortened (halving) until the grid covers the SMs once
+    // launch shape per axis: P pencils per CTA of the cross-section's rows taken
+    // one after another (as the Euler sweep's), segments shortened (halving)
+    // until the grid covers the SMs once
     void plan() {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
@@ -411,18 +412,18 @@ struct emg_five {
             }
             lane_axis[d] = lane;
             other_axis[d] = other;
-            const int64_t nd = mesh.n[d], nl = mesh.n[lane], nother = mesh.n[other];
+            const int64_t nd = mesh.n[d], pencils = mesh.n[lane] * mesh.n[other];
             int P = opts.mode == EMG_MODE_HYBRID ? 16 : 32;
-            if (nl <= 8)
+            if (pencils <= 8)
                 P = 8;
-            else if (nl <= 16)
+            else if (pencils <= 16)
                 P = 16;
-            const int64_t tiles = (nl + P - 1) / P;
+            const int64_t tiles = (pencils + P - 1) / P;
             int64_t seg = nd;
-            while (seg > 32 && tiles * ((nd + seg - 1) / seg) * nother < sms) seg = (seg + 1) / 2;
+            while (seg > 32 && tiles * ((nd + seg - 1) / seg) < sms) seg = (seg + 1) / 2;
             sweepP[d] = P;
             sweepSeg[d] = (int)seg;
-            sweepGrid[d] = dim3((unsigned)tiles, (unsigned)((nd + seg - 1) / seg), (unsigned)nother);
+            sweepGrid[d] = dim3((unsigned)tiles, (unsigned)((nd + seg - 1) / seg), 1);
         }
     }
 
@@ -688,7 +689,7 @@ int emg_five_create(const emg_mesh* mesh, const emg_five_system* sys, const emg_
         return bail(set_error(EMG_ERR_CUDA, "upload failed"));
     h->plan();
     for (int d = 0; d < 3; d++)
-        if (h->active[d] && (h->sweepGrid[d].y > 65535u || h->sweepGrid[d].z > 65535u))
+        if (h->active[d] && (h->sweepGrid[d].y > 65535u || h->mesh.n[h->other_axis[d]] > 65535))
             return bail(set_error(EMG_ERR_INVALID, "mesh too large for the sweep grid"));
     *out = h;
     return EMG_OK;

@@ -275,12 +275,11 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
             s_limited = 0;
             s_weno = 0;
         }
-        // uniform grids: x = lane tile, y = segment, z = other-axis row;
+        // uniform grids: x = tile of P pencils, y = segment;
         // AMR batches: x = (leaf, group of other-axis rows), one segment
         const int lane0 = AMR ? 0 : blockIdx.x * P;
         const int s0 = blockIdx.y * p.seg;
         int Ls = min(p.seg, p.nd - s0);
-        int ob = blockIdx.z;
         int64_t blk = 0;
         int slot_id = 0;
         double dx = p.dx;
@@ -318,8 +317,8 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                 s_pen[tid] = p.pen_lane_major ? la * p.no + ob1 : ob1 * p.nl + la;
             }
         } else if (tid < P) {
-            const int la = lane0 + tid;
-            s_lok[tid] = la < p.nl && ob < p.no;
+            const int la = (lane0 + tid) % p.nl, ob = (lane0 + tid) / p.nl;
+            s_lok[tid] = ob < p.no;
             s_loff[tid] = (int64_t)(p.gl + la) * p.sl + (int64_t)(p.go + ob) * p.so;
         }
         const int64_t base0 = blk + (int64_t)(p.gd + s0 - 5) * p.sd;

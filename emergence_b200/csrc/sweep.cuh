@@ -665,7 +665,8 @@ struct Sweep {
             // published by the lane-table barrier below
         }
 
-        // uniform grids: x = lane tile, y = segment, z = other-axis row;
+        // uniform grids: x = tile of P pencils, y = segment (TMA staging: x = lane
+        // tile of an other-axis row, z = that row);
         // AMR batches: x = (leaf, group of other-axis rows), lanes cover the block
         const int lane0 = AMR ? 0 : blockIdx.x * P;
         const int s0 = blockIdx.y * p.seg;
@@ -728,8 +729,17 @@ struct Sweep {
                 atomicMax(&s_maxlen, len);
             }
         } else if (tid < P) {
-            const int lw = AMR ? p.lw : P;
-            const int la = lane0 + tid % lw, ob = ob0 + tid / lw;
+            int la, ob;
+            if constexpr (KIND == KIND_GRID) {
+                // the cross-section's pencils in one row after another, so that
+                // only the last CTA has idle lanes
+                la = (lane0 + tid) % p.nl;
+                ob = (lane0 + tid) / p.nl;
+            } else {
+                const int lw = AMR ? p.lw : P;
+                la = lane0 + tid % lw;
+                ob = ob0 + tid / lw;
+            }
             s_lok[tid] = la < p.nl && ob < p.no;
             s_loff[tid] = (int64_t)(p.gl + la) * p.sl + (int64_t)(p.go + ob) * p.so;
             if constexpr (AMR) s_pen[tid] = p.pen_lane_major ? la * p.no + ob : ob * p.nl + la;

@@ -422,10 +422,23 @@ struct ProfScope {
     }
 };
 
-// launch grid of the sweep along d for P pencils per CTA and segments of seg cells
+// launch grid of the sweep along d for P pencils per CTA and segments of seg
+// cells: the pencils of the whole cross-section are tiled one row after
+// another, so a row length that is no multiple of P idles lanes in the last
+// CTA only (161×127×98: 12 % fewer CTAs along the two axes whose rows hold 98)
 dim3 sweep_grid(const emg_uniform* h, int d, int P, int64_t seg) {
+    const int64_t nd = h->mesh.n[d], pencils = h->mesh.n[h->lane_axis[d]] * h->mesh.n[h->other_axis[d]];
+    return dim3((unsigned)((pencils + P - 1) / P), (unsigned)((nd + seg - 1) / seg), 1);
+}
+// the TMA-staged sweep's: a box of lanes lies within one row
+static dim3 sweep_grid_rows(const emg_uniform* h, int d, int P, int64_t seg) {
     const int64_t nd = h->mesh.n[d], nl = h->mesh.n[h->lane_axis[d]], nother = h->mesh.n[h->other_axis[d]];
     return dim3((unsigned)((nl + P - 1) / P), (unsigned)((nd + seg - 1) / seg), (unsigned)nother);
+}
+// grids the launch cannot cover: more than 65535 segments, or (a limit of the
+// row-wise grid, kept for both) rows of the other axis
+static bool sweep_grid_too_large(const emg_uniform* h, int d) {
+    return h->sweepGrid[d].y > 65535u || h->mesh.n[h->other_axis[d]] > 65535;
 }
 
 // Segment length of the sweep along d: the fewest (waves of CTAs) × (rows a
@@ -434,7 +447,7 @@ dim3 sweep_grid(const emg_uniform* h, int d, int P, int64_t seg) {
 // fill the SMs on small grids, and a wave count just above a whole number is
 // avoided.
 int64_t plan_seg(const emg_uniform* h, int d, int P) {
-    const int64_t nd = h->mesh.n[d], nl = h->mesh.n[h->lane_axis[d]], nother = h->mesh.n[h->other_axis[d]];
+    const int64_t nd = h->mesh.n[d], pencils = h->mesh.n[h->lane_axis[d]] * h->mesh.n[h->other_axis[d]];
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         cudaGetLastError();
@@ -448,14 +461,14 @@ int64_t plan_seg(const emg_uniform* h, int d, int P) {
                                    : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_ctas_per_sm_fast(P, h->opts.mode)
                                                                                  : sweep_ctas_per_sm_f64(P, h->opts.mode));
     const int64_t slots = (int64_t)sms * per_sm;
-    const int64_t lane_tiles = (nl + P - 1) / P;
+    const int64_t tiles = (pencils + P - 1) / P;
     int64_t best = nd;
     double best_cost = 1e300;
     for (int64_t k = 1; k <= nd; k++) {
         const int64_t seg = (nd + k - 1) / k;
         if (k > 1 && seg < 16) break;
         if ((nd + seg - 1) / seg != k) continue;  // same seg as a smaller k
-        const int64_t ctas = lane_tiles * k * nother;
+        const int64_t ctas = tiles * k;
         if (k > 65535) break;
         const double cost = (double)((ctas + slots - 1) / slots) * (double)(seg + 6);
         if (cost < best_cost * 0.95) {  // shorter segments only for a clear gain
@@ -480,18 +493,17 @@ void plan_sweeps(emg_uniform* h) {
         }
         h->lane_axis[d] = lane;
         h->other_axis[d] = other;
-        const int64_t nd = h->mesh.n[d], nl = h->mesh.n[lane], nother = h->mesh.n[other];
+        const int64_t pencils = h->mesh.n[lane] * h->mesh.n[other];
         // hybrid rings hold RM + 9 rows: P = 16 keeps them at 2 CTAs per SM
         int P = h->opts.mode == EMG_MODE_HYBRID ? 16 : 32;
-        if (nl <= 8)
+        if (pencils <= 8)
             P = 8;
-        else if (nl <= 16)
+        else if (pencils <= 16)
             P = 16;
-        const int64_t lane_tiles = (nl + P - 1) / P;
         const int64_t seg = plan_seg(h, d, P);
         h->sweepP[d] = P;
         h->sweepSeg[d] = (int)seg;
-        h->sweepGrid[d] = dim3((unsigned)lane_tiles, (unsigned)((nd + seg - 1) / seg), (unsigned)nother);
+        h->sweepGrid[d] = sweep_grid(h, d, P, seg);
     }
 }
 
@@ -671,11 +683,11 @@ int launch_axis(emg_uniform* h, int stage, int d, double* in, bool first, bool l
         if (h->tma && h->sweepP[d] == 32 && (d != 2 || h->sweepSeg[d] % 2 == 0 || h->sweepGrid[d].y == 1))
             buf = in == h->u ? 0 : (in == h->sa ? 1 : (in == h->sb ? 2 : -1));
         cudaError_t e;
-        if (buf >= 0)
-            e = h->opts.precision == EMG_PRECISION_MIXED
-                    ? sweep_launch_tma_mixed(p, h->tmap[buf][d], h->sweepGrid[d], h->stream)
-                    : sweep_launch_tma_f64(p, h->tmap[buf][d], h->sweepGrid[d], h->stream);
-        else if (h->opts.precision == EMG_PRECISION_MIXED)
+        if (buf >= 0) {
+            const dim3 rows = sweep_grid_rows(h, d, h->sweepP[d], h->sweepSeg[d]);
+            e = h->opts.precision == EMG_PRECISION_MIXED ? sweep_launch_tma_mixed(p, h->tmap[buf][d], rows, h->stream)
+                                                         : sweep_launch_tma_f64(p, h->tmap[buf][d], rows, h->stream);
+        } else if (h->opts.precision == EMG_PRECISION_MIXED)
             e = sweep_launch_mixed(h->sweepP[d], h->opts.mode, p, h->sweepGrid[d], h->stream);
         else if (h->opts.precision == EMG_PRECISION_F64_FAST)
             e = sweep_launch_fast(h->sweepP[d], h->opts.mode, p, h->sweepGrid[d], h->stream);
@@ -733,19 +745,19 @@ int autotune_sweeps(emg_uniform* h) {
     TuneVal best{};
     for (int d = 0; d < 3; d++) {
         if (!h->active[d]) continue;
-        const int64_t nd = h->mesh.n[d], nl = h->mesh.n[h->lane_axis[d]];
+        const int64_t nd = h->mesh.n[d], pencils = h->mesh.n[h->lane_axis[d]] * h->mesh.n[h->other_axis[d]];
         float best_ms = 1e30f;
         best.P[d] = h->sweepP[d];
         best.seg[d] = h->sweepSeg[d];
         for (int P : {8, 16, 32}) {
-            if (P > 8 && nl <= P / 2) continue;                         // lanes mostly idle
+            if (P > 8 && pencils <= P / 2) continue;                         // lanes mostly idle
             if (P == 32 && h->opts.mode == EMG_MODE_HYBRID) continue;  // hybrid rings: one CTA per SM at P = 32
             const int64_t planned = plan_seg(h, d, P);
             std::set<int64_t> segs = {nd, (nd + 1) / 2, (nd + 3) / 4, planned, std::min(nd, 2 * planned), (planned + 1) / 2};
             for (int64_t seg : segs) {
                 if (seg < 16 && seg != nd) continue;
                 const dim3 g = sweep_grid(h, d, P, seg);
-                if (g.y > 65535u || g.z > 65535u) continue;
+                if (g.y > 65535u) continue;
                 h->sweepP[d] = P;
                 h->sweepSeg[d] = (int)seg;
                 h->sweepGrid[d] = g;
@@ -1062,7 +1074,7 @@ int emg_uniform_create(const emg_mesh* mesh, const emg_eos* eos, const emg_bc bc
         return bail(set_error(EMG_ERR_CUDA, "control block upload failed"));
     plan_sweeps(h);
     for (int d = 0; d < 3; d++)
-        if (h->active[d] && (h->sweepGrid[d].y > 65535u || h->sweepGrid[d].z > 65535u))
+        if (h->active[d] && sweep_grid_too_large(h, d))
             return bail(set_error(EMG_ERR_INVALID, "mesh too large for the sweep grid (an axis above 65535 pencils)"));
     setup_tma(h);
     int rc = emg_uniform_upload(h, u_aos, len);
@@ -1386,7 +1398,7 @@ int emg_uniform_step_noalloc(const emg_mesh* mesh, const emg_eos* eos, const emg
     h.u = u_out;
     plan_sweeps(&h);
     for (int d = 0; d < 3; d++)
-        if (h.active[d] && (h.sweepGrid[d].y > 65535u || h.sweepGrid[d].z > 65535u))
+        if (h.active[d] && sweep_grid_too_large(&h, d))
             return set_error(EMG_ERR_INVALID, "mesh too large for the sweep grid");
     // u_out starts as a copy of u_in; the stage kernels then work in place on
     // it (ghosts filled at stage 1, the stage-3 update written back)
