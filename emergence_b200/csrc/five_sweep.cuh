@@ -547,17 +547,27 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                     }
                 }
             }
+            // this thread's cell of phase D. Its α + K comes from the W ring before the
+            // barrier: the next round's rows overwrite those slots as soon as some
+            // warp is done with D, which no barrier follows.
+            int c, l;
+            if (p.rows_contig) {
+                c = RM * r - 5 + tid % RM;
+                l = tid / RM;
+            } else {
+                c = RM * r - 5 + tid / P;
+                l = tid % P;
+            }
+            double nc = 0.0;
+            if (s_lok[l] && c >= 0 && c < Ls) {
+                double wc[NF];
+#pragma unroll
+                for (int k = 0; k < NF; k++) wc[k] = W[at<STRW>(c + 5, k, l)];
+                nc = sys.nc_coef<FAST>(wc);
+            }
             __syncthreads();
             // ---- D: cells [RM r − 5, RM r + RM − 5)
             {
-                int c, l;
-                if (p.rows_contig) {
-                    c = RM * r - 5 + tid % RM;
-                    l = tid / RM;
-                } else {
-                    c = RM * r - 5 + tid / P;
-                    l = tid % P;
-                }
                 const int64_t g = rowg(c + 5) + s_loff[l];
                 if (s_lok[l] && c >= 0 && c < Ls && in_bounds(p.ctl, g, p.ncell)) {
                     double res[NF];
@@ -571,11 +581,8 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                     }
                     {
                         // (α + K)(Ũ⁺ − Ũ⁻)/dx of the α equation (solver.rs:440-442)
-                        double wc[NF];
-#pragma unroll
-                        for (int k = 0; k < NF; k++) wc[k] = W[at<STRW>(c + 5, k, l)];
                         const double du = F[atF(c + 1, NF, l)] - F[atF(c, NF, l)];
-                        res[F_IA] = res[F_IA] + (AMR ? sys.nc_coef<FAST>(wc) * du / dx : sys.nc_coef<FAST>(wc) * du * inv);
+                        res[F_IA] = res[F_IA] + (AMR ? nc * du / dx : nc * du * inv);
                     }
                     if (!p.last) {
 #pragma unroll
