@@ -135,7 +135,7 @@ __global__ void five_cfl_kernel(const FiveCflParams p) {
         for (int k = 0; k < NF; k++)
             if (!isfinite(w[k])) bad = 1;
         if (!(Five::rho(w) > 0.0)) bad = 1;
-        const double cs = Five::sound_speed_rc2(w, rc2);
+        const double cs = s.sound_speed_rc2(w, rc2);
         double acc = -0.0;
         for (int d = 0; d < 3; d++)
             if (p.act[d]) acc = acc + (fabs(w[F_IU + d]) + cs) / p.dx[d];

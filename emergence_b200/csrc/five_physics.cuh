@@ -9,6 +9,7 @@
 // non-zero terms of the reference's dense loops.
 #pragma once
 #include "physics.cuh"
+#include "quotient.cuh"
 
 namespace emg {
 
@@ -20,36 +21,66 @@ struct FiveSysD {
     int kapila;
 };
 
-// a/b: correctly rounded in the plain form, a·(1/b) with the one-ulp
-// reciprocal of physics.cuh in the fast FP64 form (F)
-template <bool F> __device__ __forceinline__ double fdiv(double a, double b) {
-    if constexpr (F)
-        return a * rcp_f(b);
-    else
-        return a / b;
-}
-template <bool F> __device__ __forceinline__ double fsqrt(double x) {
-    if constexpr (F)
-        return sqrt_f(x);
-    else
-        return sqrt(x);
-}
+// Forms of the closure arithmetic: the compiler's division (every operand), the
+// fast FP64 form (one-ulp reciprocals, 1/(γ − 1) of each phase precomputed), and
+// the plain form's usual path, whose branch-free quotients and square roots
+// (quotient.cuh) round as FORM_DIV does and raise Five::bad for operands outside
+// their ranges; the caller then evaluates again with FORM_DIV.
+enum FiveForm { FORM_DIV = 0, FORM_FAST = 1, FORM_RN = 2 };
 
-// Methods templated on F: the plain form (F false, the reference's operation
-// order, bit-exact without FMA contraction) or the fast FP64 form (F true,
-// one-ulp reciprocals and square roots, 1/(γ − 1) of each phase precomputed).
+__device__ __forceinline__ bool finite_bits(double x) { return (hi_bits(x) & 0x7ff00000u) != 0x7ff00000u; }
+
+// Methods templated on the form F; FORM_DIV and FORM_RN keep the reference's
+// operation order (bit-exact without FMA contraction).
 struct Five {
     Eos<double> e1, e2;
     bool kapila;
-    double igm[2];  // 1/(γ − 1) of each phase (fast form)
+    double igm[2];     // 1/(γ − 1) of each phase
+    bool gm_out;       // FORM_RN: a γ − 1 outside the branch-free range
+    mutable bool bad;  // FORM_RN: an operand left the ranges since begin()
     __device__ static Five from(const FiveSysD& s) {
         return Five{Eos<double>::from(s.e[0]), Eos<double>::from(s.e[1]), s.kapila != 0,
-                    {1.0 / (s.e[0].gamma - 1.0), 1.0 / (s.e[1].gamma - 1.0)}};
+                    {1.0 / (s.e[0].gamma - 1.0), 1.0 / (s.e[1].gamma - 1.0)},
+                    den_out(s.e[0].gamma - 1.0) || den_out(s.e[1].gamma - 1.0), false};
+    }
+    __device__ __forceinline__ void begin() const { bad = gm_out; }
+    // a/b, b > 0 (any b in FORM_DIV)
+    template <int F> __device__ __forceinline__ double div(double a, double b) const {
+        if constexpr (F == FORM_FAST)
+            return a * rcp_f(b);
+        else if constexpr (F == FORM_RN)
+            return div_rn(a, den_rn(b, bad), bad);
+        else
+            return a / b;
+    }
+    // a/b, b of either sign
+    template <int F> __device__ __forceinline__ double div_signed(double a, double b) const {
+        if constexpr (F == FORM_RN)
+            return div_signed_rn(a, b, bad);
+        else
+            return div<F>(a, b);
+    }
+    // a/(γ_k − 1)
+    template <int F> __device__ __forceinline__ double div_gm(double a, int k) const {
+        if constexpr (F == FORM_FAST)
+            return a * igm[k];
+        else if constexpr (F == FORM_RN)
+            return div_rn(a, RecipRn{eos(k).gamma - 1.0, igm[k]}, bad);
+        else
+            return a / (eos(k).gamma - 1.0);
+    }
+    template <int F> __device__ __forceinline__ double root(double x) const {
+        if constexpr (F == FORM_FAST)
+            return sqrt_f(x);
+        else if constexpr (F == FORM_RN)
+            return sqrt_rn(x, bad);
+        else
+            return sqrt(x);
     }
     __device__ __forceinline__ const Eos<double>& eos(int k) const { return k == 0 ? e1 : e2; }
 
     // multiphase.rs:58-69
-    template <bool F = false> __device__ __forceinline__ void db(const double* w, double& d, double& b) const {
+    template <int F = FORM_DIV> __device__ __forceinline__ void db(const double* w, double& d, double& b) const {
         const double al[2] = {w[F_IA], 1.0 - w[F_IA]};
         d = 0.0;
         b = 0.0;
@@ -57,13 +88,8 @@ struct Five {
         for (int k = 0; k < 2; k++) {
             const Eos<double>& e = eos(k);
             const double vol = al[k] - e.b * w[k];
-            if constexpr (F) {
-                d = d + vol * igm[k];
-                b = b + e.gamma * e.p_inf * vol * igm[k] + e.q * w[k];
-            } else {
-                d = d + vol / (e.gamma - 1.0);
-                b = b + e.gamma * e.p_inf * vol / (e.gamma - 1.0) + e.q * w[k];
-            }
+            d = d + div_gm<F>(vol, k);
+            b = b + div_gm<F>(e.gamma * e.p_inf * vol, k) + e.q * w[k];
         }
     }
     __device__ __forceinline__ double rho_e(const double* w) const {
@@ -72,15 +98,19 @@ struct Five {
         return w[F_IP] * d + b;
     }
     // multiphase.rs:77-84
-    template <bool F = false> __device__ __forceinline__ double rho_c2_phase(const double* w, int k) const {
+    template <int F = FORM_DIV> __device__ __forceinline__ double rho_c2_phase(const double* w, int k) const {
         const double al = k == 0 ? w[F_IA] : 1.0 - w[F_IA];
         const Eos<double>& e = eos(k);
-        if (F && e.b == 0.0) return e.gamma * (w[F_IP] + e.p_inf);  // fmax(1 − 0, 1e-12) = 1
-        const double rk = (al > 1e-12 && w[k] > 0.0) ? fdiv<F>(w[k], al) : 0.0;
-        return fdiv<F>(e.gamma * (w[F_IP] + e.p_inf), fmax(1.0 - e.b * rk, 1e-12));
+        if (F != FORM_DIV && e.b == 0.0) {  // fmax(1 − 0·rk, 1e-12) = 1 for a finite rk
+            if (F == FORM_RN) bad = bad || num_out(w[k]);
+            return e.gamma * (w[F_IP] + e.p_inf);
+        }
+        const bool has = al > 1e-12 && w[k] > 0.0;
+        const double rk = has ? div<F>(w[k], has ? al : 1.0) : 0.0;
+        return div<F>(e.gamma * (w[F_IP] + e.p_inf), fmax(1.0 - e.b * rk, 1e-12));
     }
     // multiphase.rs:86-97 (Rust clamp: NaN stays NaN)
-    template <bool F = false> __device__ __forceinline__ double kapila_k(const double* w) const {
+    template <int F = FORM_DIV> __device__ __forceinline__ double kapila_k(const double* w) const {
         if (!kapila) return 0.0;
         double a = w[F_IA];
         if (a < 0.0) a = 0.0;
@@ -89,32 +119,26 @@ struct Five {
         const double z1 = rho_c2_phase<F>(w, 0), z2 = rho_c2_phase<F>(w, 1);
         const double den = al1 * z1 + al0 * z2;
         if (den <= 0.0) return 0.0;
-        return fdiv<F>(al0 * al1 * (z2 - z1), den);
+        return div<F>(al0 * al1 * (z2 - z1), den);
     }
     // multiphase.rs:113-117
-    template <bool F = false> __device__ __forceinline__ double drhoe_dalpha(double p) const {
-        if constexpr (F)
-            return (p + e1.gamma * e1.p_inf) * igm[0] - (p + e2.gamma * e2.p_inf) * igm[1];
-        else
-            return (p + e1.gamma * e1.p_inf) / (e1.gamma - 1.0) - (p + e2.gamma * e2.p_inf) / (e2.gamma - 1.0);
+    template <int F = FORM_DIV> __device__ __forceinline__ double drhoe_dalpha(double p) const {
+        return div_gm<F>(p + e1.gamma * e1.p_inf, 0) - div_gm<F>(p + e2.gamma * e2.p_inf, 1);
     }
     // multiphase.rs:100-110, from the closure values d, b of w and K = kapila_k(w)
     // (every term as the reference evaluates it; the reference recomputes d and
     // b inside rho_e, which gives the same values)
-    template <bool F = false>
+    template <int F = FORM_DIV>
     __device__ __forceinline__ double rho_c2_db(const double* w, double d, double b, double kk) const {
         const double p = w[F_IP];
         double num = (w[F_IP] * d + b) + p;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const Eos<double>& e = eos(k);
-            if constexpr (F)
-                num = num + w[k] * (e.b * (p + e.gamma * e.p_inf) * igm[k] - e.q);
-            else
-                num = num + w[k] * (e.b * (p + e.gamma * e.p_inf) / (e.gamma - 1.0) - e.q);
+            num = num + w[k] * (div_gm<F>(e.b * (p + e.gamma * e.p_inf), k) - e.q);
         }
         num = num + kk * drhoe_dalpha<F>(p);
-        return fdiv<F>(num, d);
+        return div<F>(num, d);
     }
     __device__ __forceinline__ double rho_c2(const double* w) const {
         double d, b;
@@ -126,7 +150,7 @@ struct Five {
     struct St {
         double d, b, rc2;
     };
-    template <bool F = false> __device__ __forceinline__ St state(const double* w) const {
+    template <int F = FORM_DIV> __device__ __forceinline__ St state(const double* w) const {
         St st;
         db<F>(w, st.d, st.b);
         st.rc2 = rho_c2_db<F>(w, st.d, st.b, kapila_k<F>(w));
@@ -142,15 +166,20 @@ struct Five {
     }
     // multiphase.rs:131-146; d, b: the closure values of the result (db does
     // not read the pressure)
-    template <bool F = false>
+    template <int F = FORM_DIV>
     __device__ __forceinline__ void to_prim_db(const double* u, double* w, double& d, double& b) const {
         const double r = u[0] + u[1];
         double vx, vy, vz;
-        if constexpr (F) {
+        if constexpr (F == FORM_FAST) {
             const double ir = rcp_f(r);
             vx = u[2] * ir;
             vy = u[3] * ir;
             vz = u[4] * ir;
+        } else if constexpr (F == FORM_RN) {
+            const RecipRn ir = den_rn(r, bad);
+            vx = div_rn(u[2], ir, bad);
+            vy = div_rn(u[3], ir, bad);
+            vz = div_rn(u[4], ir, bad);
         } else {
             vx = u[2] / r;
             vy = u[3] / r;
@@ -164,7 +193,7 @@ struct Five {
         w[F_IA] = u[6];
         const double rhoe = u[5] - 0.5 * r * (vx * vx + vy * vy + vz * vz);
         db<F>(w, d, b);
-        w[F_IP] = fdiv<F>(rhoe - b, d);
+        w[F_IP] = div<F>(rhoe - b, d);
     }
     __device__ __forceinline__ void to_prim(const double* u, double* w) const {
         double d, b;
@@ -181,20 +210,21 @@ struct Five {
         u[5] = (w[F_IP] * d + b) + 0.5 * r * (w[2] * w[2] + w[3] * w[3] + w[4] * w[4]);
         u[6] = w[F_IA];
     }
-    template <bool F = false> __device__ __forceinline__ void to_cons(const double* w, double* u) const {
+    template <int F = FORM_DIV> __device__ __forceinline__ void to_cons(const double* w, double* u) const {
         double d, b;
         db<F>(w, d, b);
         to_cons_db(w, d, b, u);
     }
-    template <bool F = false> __device__ __forceinline__ static double sound_speed_rc2(const double* w, double rc2) {
-        return fsqrt<F>(fdiv<F>(fmax(rc2, 0.0), rho(w)));
+    template <int F = FORM_DIV> __device__ __forceinline__ double sound_speed_rc2(const double* w, double rc2) const {
+        // FORM_RN: root refuses what is not a positive number, so no max
+        return root<F>(div<F>(F == FORM_RN ? rc2 : fmax(rc2, 0.0), rho(w)));
     }
     __device__ __forceinline__ double sound_speed(const double* w) const { return sound_speed_rc2(w, rho_c2(w)); }
     // multiphase.rs:345-350, with ρc² of w
     __device__ __forceinline__ static bool admissible_rc2(const double* w, double rc2) {
 #pragma unroll
         for (int k = 0; k < NF; k++)
-            if (!isfinite(w[k])) return false;
+            if (!finite_bits(w[k])) return false;
         return rho(w) > 0.0 && w[F_IA] >= -0.05 && w[F_IA] <= 1.05 && rc2 > 0.0;
     }
     __device__ __forceinline__ bool admissible(const double* w) const { return admissible_rc2(w, rho_c2(w)); }
@@ -209,7 +239,7 @@ struct Five {
     }
     // multiphase.rs:245-289 (HLLC, Davis bounds) with the closure values of
     // both states; returns the contact speed
-    template <bool F = false>
+    template <int F = FORM_DIV>
     __device__ __forceinline__ double riemann_st(const double* wl, const double* wr, const St& stl, const St& str_,
                                                  int un, double* f) const {
         const double cl = sound_speed_rc2<F>(wl, stl.rc2), cr = sound_speed_rc2<F>(wr, str_.rc2);
@@ -229,15 +259,19 @@ struct Five {
         }
         const double rl = rho(wl), rr = rho(wr);
         const double pl = wl[F_IP], pr = wr[F_IP];
-        const double ss = fdiv<F>(pr - pl + rl * ul * (sl - ul) - rr * ur * (sr - ur), rl * (sl - ul) - rr * (sr - ur));
+        const double ss = div_signed<F>(pr - pl + rl * ul * (sl - ul) - rr * ur * (sr - ur), rl * (sl - ul) - rr * (sr - ur));
         const bool left = ss >= 0.0;
-        const double* w = left ? wl : wr;
-        const double* q = left ? ql : qr;
+        double w[NF], q[NF];
+#pragma unroll
+        for (int k = 0; k < NF; k++) {
+            w[k] = left ? wl[k] : wr[k];
+            q[k] = left ? ql[k] : qr[k];
+        }
         const double s = left ? sl : sr;
         double fx[NF];
         flux_wq(w, q, un, fx);
         const double rh = rho(w), u = w[un];
-        const double fac = fdiv<F>(s - u, s - ss);
+        const double fac = div_signed<F>(s - u, s - ss);
         double qs[NF];
         qs[0] = w[0] * fac;
         qs[1] = w[1] * fac;
@@ -245,7 +279,7 @@ struct Five {
         qs[3] = rh * fac * w[3];
         qs[4] = rh * fac * w[4];
         qs[un] = rh * fac * ss;
-        qs[5] = rh * fac * (fdiv<F>(q[5], rh) + (ss - u) * (ss + fdiv<F>(w[F_IP], rh * (s - u))));
+        qs[5] = rh * fac * (div<F>(q[5], rh) + (ss - u) * (ss + div_signed<F>(w[F_IP], rh * (s - u))));
         qs[6] = w[F_IA] * fac;
 #pragma unroll
         for (int k = 0; k < NF; k++) f[k] = fx[k] + s * (qs[k] - q[k]);
@@ -254,7 +288,7 @@ struct Five {
     __device__ __forceinline__ double riemann(const double* wl, const double* wr, int un, double* f) const {
         return riemann_st(wl, wr, state(wl), state(wr), un, f);
     }
-    template <bool F = false> __device__ __forceinline__ double nc_coef(const double* w) const {
+    template <int F = FORM_DIV> __device__ __forceinline__ double nc_coef(const double* w) const {
         return w[F_IA] + kapila_k<F>(w);
     }
     // multiphase.rs:363-377, with ρc² of w

@@ -83,7 +83,8 @@ template <int P, int MODE> struct FiveSmem {
 };
 
 // FAST: the fast FP64 form (built with FMA contraction, WENO5-Z weights from
-// the one-ulp reciprocals of physics.cuh's fast section)
+// the one-ulp reciprocals of physics.cuh's fast section); otherwise the plain
+// form, FORM_RN with FORM_DIV behind it
 template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct FiveSweep {
     using SM = FiveSmem<P, MODE>;
     static constexpr int T = SWEEP_THREADS;
@@ -106,7 +107,12 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
         return (int)((unsigned)x % (unsigned)SM::RSF) * STR + k * P + l;
     }
 
-    // scheme.rs:286-333 with the five-equation eigenvectors (multiphase.rs:202-236)
+    // the form of the sweep's usual path; FORM_RN falls back to FORM_DIV
+    static constexpr int FORM = FAST ? FORM_FAST : FORM_RN;
+
+    // scheme.rs:286-333 with the five-equation eigenvectors (multiphase.rs:202-236).
+    // FORM_RN: the result counts only if s.bad is clear afterwards.
+    template <int F>
     __device__ static __forceinline__ double midpoint(const Five& s, const double* __restrict__ W, int m, int l,
                                                       double* f, bool& fb) {
         const int j = m + 2;
@@ -114,17 +120,17 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
 #pragma unroll
         for (int k = 0; k < NF; k++) avg[k] = 0.5 * (W[at<STRW>(j, k, l)] + W[at<STRW>(j + 1, k, l)]);
         const double rh = Five::rho(avg);
-        const double kk = s.kapila_k<FAST>(avg);
+        const double kk = s.kapila_k<F>(avg);
         double c;
         {
             double d, b;
-            s.db<FAST>(avg, d, b);
-            c = Five::sound_speed_rc2<FAST>(avg, s.rho_c2_db<FAST>(avg, d, b, kk));
+            s.db<F>(avg, d, b);
+            c = s.sound_speed_rc2<F>(avg, s.rho_c2_db<F>(avg, d, b, kk));
         }
         const double c2 = c * c;
         double l0p, l1p, l2u, l2p, l5u, l5p, l6p;  // rows of L (multiphase.rs:202-220)
         double r0, r1, ru2, ru5, r6;               // columns of R (multiphase.rs:222-236)
-        if constexpr (FAST) {
+        if constexpr (F == FORM_FAST) {
             const double irh = rcp_f(rh), ic = rcp_f(c), ic2 = ic * ic;
             l0p = -avg[0] * irh * ic2;
             l1p = -avg[1] * irh * ic2;
@@ -138,6 +144,22 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
             ru2 = -c * irh;
             ru5 = c * irh;
             r6 = -kk * irh;
+        } else if constexpr (F == FORM_RN) {
+            // the quotients below; by 2c and 2c² as halves of those by c and c² (exact)
+            const RecipRn irh = den_rn(rh, s.bad), ic = den_rn(c, s.bad), ic2 = den_rn(c2, s.bad);
+            r0 = div_rn(avg[0], irh, s.bad);
+            r1 = div_rn(avg[1], irh, s.bad);
+            const double kr = div_rn(kk, irh, s.bad);
+            l0p = -div_rn(r0, ic2, s.bad);
+            l1p = -div_rn(r1, ic2, s.bad);
+            l5u = 0.5 * div_rn(rh, ic, s.bad);
+            l2u = -l5u;
+            l2p = 0.5 * ic2.y;
+            l5p = l2p;
+            l6p = div_rn(kr, ic2, s.bad);
+            ru5 = quot_rn(c, irh);
+            ru2 = -ru5;
+            r6 = -kr;
         } else {
             l0p = -avg[0] / rh / c2;
             l1p = -avg[1] / rh / c2;
@@ -169,7 +191,9 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                     default: ch[s6] = l6p * W[at<STRW>(row, F_IP, l)] + W[at<STRW>(row, F_IA, l)];
                 }
             }
-            if constexpr (FAST) {
+            if constexpr (F == FORM_RN) {
+                weno5z_pair_rn(ch, cl[a], cr[a], s.bad);
+            } else if constexpr (F == FORM_FAST) {
                 cl[a] = weno5z_interp_f(ch[0], ch[1], ch[2], ch[3], ch[4]);
                 cr[a] = weno5z_interp_f(ch[5], ch[4], ch[3], ch[2], ch[1]);
             } else {
@@ -194,7 +218,8 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
         wl[F_IA] = (r6 * cl[2] + r6 * cl[5]) + cl[6];
         wr[F_IA] = (r6 * cr[2] + r6 * cr[5]) + cr[6];
         fb = false;
-        Five::St stl = s.state<FAST>(wl), str_ = s.state<FAST>(wr);
+        if (F == FORM_RN && s.bad) return 0.0;
+        Five::St stl = s.state<F>(wl), str_ = s.state<F>(wr);
         if (!Five::admissible_rc2(wl, stl.rc2) || !Five::admissible_rc2(wr, str_.rc2)) {
             fb = true;
 #pragma unroll
@@ -202,11 +227,77 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                 wl[k] = W[at<STRW>(j, k, l)];
                 wr[k] = W[at<STRW>(j + 1, k, l)];
             }
-            stl = s.state<FAST>(wl);
-            str_ = s.state<FAST>(wr);
+            stl = s.state<F>(wl);
+            str_ = s.state<F>(wr);
         }
-        return s.riemann_st<FAST>(wl, wr, stl, str_, UN, f);
+        return s.riemann_st<F>(wl, wr, stl, str_, UN, f);
     }
+
+    // the same midpoint with the compiler's division, straight into the flux ring
+    __device__ static __noinline__ bool midpoint_div(const Five s, const double* __restrict__ W, double* MF, int m, int l) {
+        double f[NF];
+        bool fb;
+        const double us = midpoint<FORM_DIV>(s, W, m, l, f, fb);
+#pragma unroll
+        for (int k = 0; k < NF; k++) MF[atM(m, k, l)] = f[k];
+        MF[atM(m, NF, l)] = us;
+        return fb;
+    }
+    // maps of the usual path, evaluated again with FORM_DIV where they must be
+    // (operands by value, so that the caller's stay in registers)
+    struct State {
+        double v[NF];
+    };
+    struct PrimDb {
+        double w[NF], d, b;
+    };
+    __device__ static __forceinline__ State pack(const double* u) {
+        State x;
+#pragma unroll
+        for (int k = 0; k < NF; k++) x.v[k] = u[k];
+        return x;
+    }
+    __device__ static __noinline__ PrimDb prim_div(const Five s, const State u) {
+        PrimDb r;
+        s.to_prim_db<FORM_DIV>(u.v, r.w, r.d, r.b);
+        return r;
+    }
+    __device__ static __forceinline__ void to_prim(const Five& s, const double* u, double* w, double& d, double& b) {
+        s.begin();
+        s.to_prim_db<FORM>(u, w, d, b);
+        if (FORM == FORM_RN && s.bad) {
+            const PrimDb r = prim_div(s, pack(u));
+#pragma unroll
+            for (int k = 0; k < NF; k++) w[k] = r.w[k];
+            d = r.d;
+            b = r.b;
+        }
+    }
+    __device__ static __noinline__ State cons_div(const Five s, const State w) {
+        State u;
+        s.to_cons<FORM_DIV>(w.v, u.v);
+        return u;
+    }
+    __device__ static __forceinline__ void to_cons(const Five& s, const double* w, double* u) {
+        s.begin();
+        s.to_cons<FORM>(w, u);
+        if (FORM == FORM_RN && s.bad) {
+            const State r = cons_div(s, pack(w));
+#pragma unroll
+            for (int k = 0; k < NF; k++) u[k] = r.v[k];
+        }
+    }
+    __device__ static __noinline__ double nc_coef_div(const Five s, const State w) { return s.nc_coef<FORM_DIV>(w.v); }
+    __device__ static __forceinline__ double nc_coef(const Five& s, const double* w) {
+        s.begin();
+        const double x = s.nc_coef<FORM>(w);
+        return FORM == FORM_RN && s.bad ? nc_coef_div(s, pack(w)) : x;
+    }
+    __device__ static __noinline__ double div_slow(double a, double b) { return a / b; }
+    __device__ static __forceinline__ double quot_plain(double a, const RecipRn& d, bool out) {
+        return out || num_out(a) ? div_slow(a, d.b) : quot_rn(a, d);
+    }
+
 
     // KEEP-PE two-point flux with cached ρe (multiphase.rs:291-309)
     __device__ static __forceinline__ void split_flux(const double* __restrict__ W, int ra, int rb, int l, double* f) {
@@ -233,17 +324,26 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
     }
 
     // one-sided admissibility of the limiter (scheme.rs:408-416)
+    template <int F> __device__ static __forceinline__ bool side_ok(const Five& s, const double* a) {
+        double w[NF], d, b;
+        s.to_prim_db<F>(a, w, d, b);
+        return Five::admissible_rc2(w, s.rho_c2_db<F>(w, d, b, s.kapila_k<F>(w)));
+    }
+    __device__ static __noinline__ bool side_ok_div(const Five s, const State a) { return side_ok<FORM_DIV>(s, a.v); }
+    __device__ static __forceinline__ bool side_ok_any(const Five& s, const double* a) {
+        s.begin();
+        const bool ok = side_ok<FORM>(s, a);
+        return FORM == FORM_RN && s.bad ? side_ok_div(s, pack(a)) : ok;
+    }
     __device__ static __forceinline__ bool lim_ok(const Five& s, const double* fx, const double* ul, const double* fl,
                                                   const double* ur, const double* fr, double lam2) {
-        double a[NF], w[NF], d, b;
+        double a[NF];
 #pragma unroll
         for (int k = 0; k < NF; k++) a[k] = ul[k] - lam2 * (fx[k] - fl[k]);
-        s.to_prim_db<FAST>(a, w, d, b);
-        if (!Five::admissible_rc2(w, s.rho_c2_db<FAST>(w, d, b, s.kapila_k<FAST>(w)))) return false;
+        if (!side_ok_any(s, a)) return false;
 #pragma unroll
         for (int k = 0; k < NF; k++) a[k] = ur[k] + lam2 * (fx[k] - fr[k]);
-        s.to_prim_db<FAST>(a, w, d, b);
-        return Five::admissible_rc2(w, s.rho_c2_db<FAST>(w, d, b, s.kapila_k<FAST>(w)));
+        return side_ok_any(s, a);
     }
 
     __device__ static __forceinline__ double d4(double q0, double q1, double q2, double q3, double q4) {
@@ -349,6 +449,8 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
         const double lam2 = 2.0 * lam;
         const bool lim_on = p.positivity && lam > 0.0;
         const double inv = 1.0 / dx;
+        const RecipRn rdx{dx, inv}, r3{3.0, 1.0 / 3.0};
+        const bool dx_out = den_out(dx);
         __syncthreads();
         const int nrounds = (Ls + 5 + RM - 1) / RM;
         const int nrows = Ls + 10;
@@ -374,7 +476,7 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                         double u[NF], w[NF], d, b;
 #pragma unroll
                         for (int k = 0; k < NF; k++) u[k] = __ldg(p.uin + k * p.ncell + g);
-                        sys.to_prim_db<FAST>(u, w, d, b);
+                        to_prim(sys, u, w, d, b);
 #pragma unroll
                         for (int k = 0; k < NF; k++) W[at<STRW>(row, k, l)] = w[k];
                         if constexpr (MODE != MODE_WENO) W[at<STRW>(row, NF, l)] = w[F_IP] * d + b;  // ρe (multiphase.rs:71-75)
@@ -422,10 +524,15 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                     if (need) {
                         double f[NF];
                         bool fb;
-                        const double us = midpoint(sys, W, m, l, f, fb);
+                        sys.begin();
+                        const double us = midpoint<FORM>(sys, W, m, l, f, fb);
+                        if (FORM == FORM_RN && sys.bad) {
+                            fb = midpoint_div(sys, W, MF, m, l);
+                        } else {
 #pragma unroll
-                        for (int k = 0; k < NF; k++) MF[atM(m, k, l)] = f[k];
-                        MF[atM(m, NF, l)] = us;
+                            for (int k = 0; k < NF; k++) MF[atM(m, k, l)] = f[k];
+                            MF[atM(m, NF, l)] = us;
+                        }
                         if (fb && (m < Ls || tail)) atomicAdd(&s_fallback, chain_mult(m, 5));
                     }
                 }
@@ -498,13 +605,13 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                             wi[k] = W[at<STRW>(i, k, l)];
                             wj[k] = W[at<STRW>(i + 1, k, l)];
                         }
-                        sys.to_cons<FAST>(wi, ul);
-                        sys.to_cons<FAST>(wj, ur);
+                        to_cons(sys, wi, ul);
+                        to_cons(sys, wj, ur);
                         Five::flux_wq(wi, ul, UN, flp);
                         Five::flux_wq(wj, ur, UN, frp);
                         bool finite = true;
 #pragma unroll
-                        for (int k = 0; k < NF; k++) finite = finite && isfinite(fh[k]);
+                        for (int k = 0; k < NF; k++) finite = finite && finite_bits(fh[k]);
                         if (!(finite && lim_ok(sys, fh, ul, flp, ur, frp, lam2))) {
                             const double alpha = fmax(fabs(wi[UN]) + sys.sound_speed(wi), fabs(wj[UN]) + sys.sound_speed(wj));
                             double flf[NF], bl[NF];
@@ -563,7 +670,7 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                 double wc[NF];
 #pragma unroll
                 for (int k = 0; k < NF; k++) wc[k] = W[at<STRW>(c + 5, k, l)];
-                nc = sys.nc_coef<FAST>(wc);
+                nc = nc_coef(sys, wc);
             }
             __syncthreads();
             // ---- D: cells [RM r − 5, RM r + RM − 5)
@@ -575,7 +682,7 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                     for (int k = 0; k < NF; k++) {
                         // the block solver divides by dx (C/amr.rs:1273), the uniform one multiplies by 1/dx
                         const double df = F[atF(c + 1, k, l)] - F[atF(c, k, l)];
-                        const double x = AMR ? df / dx : df * inv;
+                        const double x = AMR ? (FAST ? df / dx : quot_plain(df, rdx, dx_out)) : df * inv;
                         const double prev = p.first ? 0.0 : p.rhs[k * p.ncell + g];
                         res[k] = prev - x;
                     }
@@ -597,7 +704,7 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                             else if (p.stage == 2)
                                 v = 0.75 * o + 0.25 * (p.cur[k * p.ncell + g] + dt * res[k]);
                             else
-                                v = p.cur[k * p.ncell + g] / 3.0 + (2.0 / 3.0) * (o + dt * res[k]);
+                                v = (FAST ? p.cur[k * p.ncell + g] / 3.0 : quot_plain(p.cur[k * p.ncell + g], r3, false)) + (2.0 / 3.0) * (o + dt * res[k]);
                             p.dest[k * p.ncell + g] = v;
                         }
                     }
