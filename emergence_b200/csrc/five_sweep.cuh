@@ -194,8 +194,7 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
             if constexpr (F == FORM_RN) {
                 weno5z_pair_rn(ch, cl[a], cr[a], s.bad);
             } else if constexpr (F == FORM_FAST) {
-                cl[a] = weno5z_interp_f(ch[0], ch[1], ch[2], ch[3], ch[4]);
-                cr[a] = weno5z_interp_f(ch[5], ch[4], ch[3], ch[2], ch[1]);
+                weno5z_pair_f(ch, cl[a], cr[a]);
             } else {
                 cl[a] = weno5z_interp(ch[0], ch[1], ch[2], ch[3], ch[4]);
                 cr[a] = weno5z_interp(ch[5], ch[4], ch[3], ch[2], ch[1]);

@@ -410,6 +410,82 @@ __device__ __forceinline__ double weno5z_interp_f(double v0, double v1, double v
     return (a0 * q0 + a1 * q1 + a2 * q2) * rcp_f(a0 + a1 + a2);
 }
 
+#ifdef __CUDACC__
+// Both WENO5-Z interpolations of a six-value stencil, v0..v4 to the midpoint
+// between v2 and v3 and the mirror image v5..v1, from the five differences
+// d_i = v_{i+1} − v_i and four second differences s_i, which the two sides share:
+//   4β_k = (13/3)·s² + B², B one of s ± 2d or d + d;  8(q_k − centre) = c·d + c'·d.
+// With x_k = 4(β_k + ε) and τ = |x0 − x2|, the weights d_k(1 + (τ/x_k)²) times
+// (x0·x1·x2)² need no division: d_k((x0x1x2)² + (τ·x_i·x_j)²). One reciprocal
+// per side is left, for the normalisation. 85 FP64 operations for the two
+// sides, where weno5z_interp_f twice takes 124. The sixth powers stay in range
+// for 4e-40 ≤ x < 2^150; larger (or not finite) x take weno5z_interp_f.
+__device__ __forceinline__ double weno5z_side_f(double x0, double x1, double x2, double e0, double e1, double e2,
+                                                double centre) {
+    // e0 = 8δ0, e1 = 80δ1, e2 = 40δ2: candidate minus centre, times its linear weight
+    const double tau = fabs(x0 - x2);
+    const double x01 = x0 * x1, p = x01 * x2;
+    const double u0 = tau * (x1 * x2), u1 = tau * (x0 * x2), u2 = tau * x01;
+    const double pp = p * p;
+    const double a0 = fma(u0, u0, pp), a1 = fma(u1, u1, pp), a2 = fma(u2, u2, pp);
+    const double den = fma(5.0, a2, fma(10.0, a1, a0));
+    const double num = fma(a2, e2, fma(a1, e1, a0 * e0));
+    return fma(0.125, num * rcp_f(den), centre);
+}
+__device__ __noinline__ static double weno5z_far_f(double v0, double v1, double v2, double v3, double v4) {
+    return weno5z_interp_f(v0, v1, v2, v3, v4);
+}
+__device__ __forceinline__ void weno5z_pair_f(const double* v, double& left, double& right) {
+    const double d0 = v[1] - v[0], d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3], d4 = v[5] - v[4];
+    const double s1 = d1 - d0, s2 = d2 - d1, s3 = d3 - d2, s4 = d4 - d3;
+    constexpr double C = 13.0 / 3.0, E = 4e-40;
+    const double t1 = fma(C * s1, s1, E), t2 = fma(C * s2, s2, E), t3 = fma(C * s3, s3, E), t4 = fma(C * s4, s4, E);
+    const double b0 = fma(2.0, d1, s1), b1 = d1 + d2, b2 = fma(-2.0, d2, s3);
+    const double c0 = fma(-2.0, d3, s4), c1 = d2 + d3, c2 = fma(2.0, d2, s2);
+    const double x0 = fma(b0, b0, t1), x1 = fma(b1, b1, t2), x2 = fma(b2, b2, t3);
+    const double y0 = fma(c0, c0, t4), y1 = fma(c1, c1, t3), y2 = fma(c2, c2, t2);
+    left = weno5z_side_f(x0, x1, x2, fma(7.0, d1, -3.0 * d0), fma(30.0, d2, 10.0 * d1), fma(25.0, d2, -5.0 * d3), v[2]);
+    right = weno5z_side_f(y0, y1, y2, fma(-7.0, d3, 3.0 * d4), fma(-30.0, d2, -10.0 * d3), fma(-25.0, d2, 5.0 * d1), v[3]);
+    // x ≥ 4e-40 > 0, so the high words order the values; NaN and infinities lie above
+    const unsigned m = max(max(max((unsigned)__double2hiint(x0), (unsigned)__double2hiint(x1)), (unsigned)__double2hiint(x2)),
+                           max(max((unsigned)__double2hiint(y0), (unsigned)__double2hiint(y1)), (unsigned)__double2hiint(y2)));
+    if (m >= (1023u + 150u) << 20) {
+        left = weno5z_far_f(v[0], v[1], v[2], v[3], v[4]);
+        right = weno5z_far_f(v[5], v[4], v[3], v[2], v[1]);
+    }
+}
+
+// The mixed form's pair: the five differences formed in FP64 and rounded to
+// FP32 once for both sides, the rest in FP32 as above; the weights as in
+// weno5z_interp<float> (scaled so that a flat stencil does not overflow); the
+// correction to the centre is added in FP64.
+__device__ __forceinline__ float weno5z_side_m(float x0, float x1, float x2, float e0, float e1, float e2) {
+    const float tau = fabsf(x0 - x2);
+    const float m = fminf(x0, fminf(x1, x2));
+    const float it = 1.0f / fmaxf(tau, m);
+    const float g = m * it, h = tau * it;
+    const float r0 = (m / x0) * h, r1 = (m / x1) * h, r2 = (m / x2) * h;
+    const float g2 = g * g;
+    const float a0 = fmaf(r0, r0, g2), a1 = fmaf(r1, r1, g2), a2 = fmaf(r2, r2, g2);
+    const float den = fmaf(5.0f, a2, fmaf(10.0f, a1, a0));
+    const float num = fmaf(a2, e2, fmaf(a1, e1, a0 * e0));
+    return num / (8.0f * den);
+}
+__device__ __forceinline__ void weno5z_pair_m(const double* v, double& left, double& right) {
+    const float d0 = (float)(v[1] - v[0]), d1 = (float)(v[2] - v[1]), d2 = (float)(v[3] - v[2]), d3 = (float)(v[4] - v[3]),
+                d4 = (float)(v[5] - v[4]);
+    const float s1 = d1 - d0, s2 = d2 - d1, s3 = d3 - d2, s4 = d4 - d3;
+    constexpr float C = 13.0f / 3.0f, E = 4e-30f;
+    const float t1 = fmaf(C * s1, s1, E), t2 = fmaf(C * s2, s2, E), t3 = fmaf(C * s3, s3, E), t4 = fmaf(C * s4, s4, E);
+    const float b0 = fmaf(2.0f, d1, s1), b1 = d1 + d2, b2 = fmaf(-2.0f, d2, s3);
+    const float c0 = fmaf(-2.0f, d3, s4), c1 = d2 + d3, c2 = fmaf(2.0f, d2, s2);
+    left = v[2] + (double)weno5z_side_m(fmaf(b0, b0, t1), fmaf(b1, b1, t2), fmaf(b2, b2, t3), fmaf(7.0f, d1, -3.0f * d0),
+                                        fmaf(30.0f, d2, 10.0f * d1), fmaf(25.0f, d2, -5.0f * d3));
+    right = v[3] + (double)weno5z_side_m(fmaf(c0, c0, t4), fmaf(c1, c1, t3), fmaf(c2, c2, t2), fmaf(-7.0f, d3, 3.0f * d4),
+                                         fmaf(-30.0f, d2, -10.0f * d3), fmaf(-25.0f, d2, 5.0f * d1));
+}
+#endif
+
 // Coefficients of the 6th-order schemes (scheme.rs:88-92).
 __device__ __forceinline__ double s6(int s) {
     return s == 0 ? (75.0 / 64.0 - 25.0 / 384.0 + 3.0 / 640.0) : (s == 1 ? (-25.0 / 384.0 + 3.0 / 640.0) : 3.0 / 640.0);

@@ -407,11 +407,7 @@ struct Sweep {
                     default: ch[s2] = l4un * Wd[at<STRW>(row, un, l)] + l04 * Wd[at<STRW>(row, 4, l)];
                 }
             }
-            const double bl = ch[2], br = ch[3];
-            cl[a] = bl + (double)weno5z_interp<float>((float)(ch[0] - bl), (float)(ch[1] - bl), 0.0f, (float)(ch[3] - bl),
-                                                      (float)(ch[4] - bl));
-            cr[a] = br + (double)weno5z_interp<float>((float)(ch[5] - br), (float)(ch[4] - br), 0.0f, (float)(ch[2] - br),
-                                                      (float)(ch[1] - br));
+            weno5z_pair_m(ch, cl[a], cr[a]);
         }
         double wl[5], wr[5];
         wl[0] = (cl[0] + cl[1]) + cl[4];
@@ -474,8 +470,7 @@ struct Sweep {
                     default: ch[s2] = l4un * Wd[at<STRW>(row, un, l)] + l04 * Wd[at<STRW>(row, 4, l)];
                 }
             }
-            cl[a] = weno5z_interp_f(ch[0], ch[1], ch[2], ch[3], ch[4]);
-            cr[a] = weno5z_interp_f(ch[5], ch[4], ch[3], ch[2], ch[1]);
+            weno5z_pair_f(ch, cl[a], cr[a]);
         }
         double wl[5], wr[5];
         wl[0] = (cl[0] + cl[1]) + cl[4];
