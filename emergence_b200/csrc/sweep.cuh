@@ -162,8 +162,8 @@ template <int RM, int MODE> struct RingSize {
     static constexpr int value = need <= 16 ? 16 : (need <= 32 ? 32 : (need <= 64 ? 64 : 128));
 };
 
-template <typename RF, int P, int MODE> struct SweepSmem {
-    static constexpr int RM = SWEEP_THREADS / P;
+template <typename RF, int P, int MODE, int T = SWEEP_THREADS> struct SweepSmem {
+    static constexpr int RM = T / P;
     static constexpr int RS = RingSize<RM, MODE>::value;  // W (and TH) ring rows
     // the flux rings hold exactly what one round keeps alive: phase C of round
     // r reads midpoints [RM r − 4, RM r + RM) and phase D faces [RM r − 5,
@@ -191,6 +191,18 @@ template <typename RF, int P, int MODE> struct SweepSmem {
 // round ahead into a shared-memory staging buffer) instead of per-thread loads.
 enum SweepKind { KIND_GRID = 0, KIND_AMR = 1, KIND_BATCH = 2, KIND_GRID_TMA = 3 };
 
+// Threads per CTA. The fast and mixed forms' WENO sweeps of uniform grids run
+// CTAs of 128 threads over 16 pencils, 8 rows a round as the 256-thread CTAs of
+// 32: half as many warps meet at each of the four barriers of a round, and the
+// SM has twice as many CTAs in other phases to fill the gap. Fast form,
+// 161×127×98, 12 steps: 28.1 → 26.8 ms (5 CTAs, 96 registers); mixed, 192³,
+// 8 steps: 57.2 → 53.1 ms (6 CTAs, 80 registers). The plain form's sweeps,
+// whose phase B is twice as long, lose (256³: 128.7 → 130.4 ms), as do the
+// 16-cell AMR blocks, which 16 rows a round cross in fewer rounds.
+template <typename RF, int MODE, int KIND> constexpr int sweep_threads() {
+    return (RingTypes<RF>::FAST || RingTypes<RF>::MIXED) && MODE == MODE_WENO && KIND == KIND_GRID ? 128 : SWEEP_THREADS;
+}
+
 // Staging buffer of KIND_GRID_TMA (bytes, plus 128 for its alignment).
 template <int P> constexpr size_t tma_stage_bytes() { return (size_t)5 * P * (SWEEP_THREADS / P) * sizeof(double) + 128; }
 
@@ -199,8 +211,8 @@ struct Sweep {
     static constexpr bool AMR = KIND == KIND_AMR;
     static constexpr bool BATCH = KIND == KIND_BATCH;
     static constexpr bool TMA = KIND == KIND_GRID_TMA;
-    using SM = SweepSmem<RF, P, MODE>;
-    static constexpr int T = SWEEP_THREADS;
+    static constexpr int T = sweep_threads<RF, MODE, KIND>();
+    using SM = SweepSmem<RF, P, MODE, T>;
     static constexpr int RM = T / P;
     static constexpr int RS = SM::RS;
     static constexpr int STR = SM::STR;

@@ -8,8 +8,13 @@
 
 namespace emg {
 
+// dynamic shared memory of the uniform-grid kernel
+template <int P, int MODE> constexpr size_t grid_smem() {
+    return SweepSmem<F64Fast, P, MODE, sweep_threads<F64Fast, MODE, KIND_GRID>()>::bytes();
+}
+
 template <int P, int D, int MODE, int KIND = KIND_GRID>
-__global__ void __launch_bounds__(SWEEP_THREADS, 3) sweep_fast_kernel(const SweepParams p) {
+__global__ void __launch_bounds__(sweep_threads<F64Fast, MODE, KIND>(), sweep_threads<F64Fast, MODE, KIND>() == 128 ? 5 : 3) sweep_fast_kernel(const SweepParams p) {
     Sweep<F64Fast, P, D, MODE, KIND>::run(p);
 }
 
@@ -48,7 +53,8 @@ cudaError_t sweep_launch_amr_fast(int P, int mode, const SweepParams& p, dim3 gr
 }
 
 template <int P, int D, int MODE> static cudaError_t launch(const SweepParams& p, dim3 grid, cudaStream_t s) {
-    sweep_fast_kernel<P, D, MODE><<<grid, SWEEP_THREADS, SweepSmem<F64Fast, P, MODE>::bytes(), s>>>(p);
+    constexpr int T = sweep_threads<F64Fast, MODE, KIND_GRID>();
+    sweep_fast_kernel<P, D, MODE><<<grid, T, grid_smem<P, MODE>(), s>>>(p);
     return cudaGetLastError();
 }
 
@@ -75,10 +81,10 @@ cudaError_t sweep_launch_fast(int P, int mode, const SweepParams& p, dim3 grid, 
 }
 
 template <int P, int MODE> static cudaError_t attr_d() {
-    const int b = (int)SweepSmem<F64Fast, P, MODE>::bytes();
-    cudaError_t e = cudaFuncSetAttribute(sweep_fast_kernel<P, 0, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fast_kernel<P, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fast_kernel<P, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    const int g = (int)grid_smem<P, MODE>(), b = (int)SweepSmem<F64Fast, P, MODE>::bytes();
+    cudaError_t e = cudaFuncSetAttribute(sweep_fast_kernel<P, 0, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, g);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fast_kernel<P, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, g);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fast_kernel<P, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, g);
     if constexpr (P >= 16) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fast_kernel<P, 0, MODE, KIND_AMR>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_fast_kernel<P, 1, MODE, KIND_AMR>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
@@ -112,8 +118,8 @@ cudaError_t sweep_prepare_fast() {
 // resident CTAs per SM of the uniform-grid sweep (the three axes share registers and shared memory)
 template <int P, int MODE> static int occupancy() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_fast_kernel<P, 0, MODE>, SWEEP_THREADS,
-                                                      SweepSmem<F64Fast, P, MODE>::bytes()) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_fast_kernel<P, 0, MODE>, sweep_threads<F64Fast, MODE, KIND_GRID>(),
+                                                      grid_smem<P, MODE>()) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }

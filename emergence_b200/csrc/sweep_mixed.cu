@@ -5,8 +5,13 @@
 
 namespace emg {
 
+// dynamic shared memory of the uniform-grid kernel
+template <int P, int MODE> constexpr size_t grid_smem() {
+    return SweepSmem<float, P, MODE, sweep_threads<float, MODE, KIND_GRID>()>::bytes();
+}
+
 template <int P, int D, int MODE, int KIND = KIND_GRID>
-__global__ void __launch_bounds__(SWEEP_THREADS, 4) sweep_mixed_kernel(const SweepParams p) {
+__global__ void __launch_bounds__(sweep_threads<float, MODE, KIND>(), sweep_threads<float, MODE, KIND>() == 128 ? 6 : 3) sweep_mixed_kernel(const SweepParams p) {
     Sweep<float, P, D, MODE, KIND>::run(p);
 }
 
@@ -31,7 +36,8 @@ cudaError_t sweep_launch_amr_mixed(int P, int mode, const SweepParams& p, dim3 g
 }
 
 template <int P, int D, int MODE> static cudaError_t launch(const SweepParams& p, dim3 grid, cudaStream_t s) {
-    sweep_mixed_kernel<P, D, MODE><<<grid, SWEEP_THREADS, SweepSmem<float, P, MODE>::bytes(), s>>>(p);
+    constexpr int T = sweep_threads<float, MODE, KIND_GRID>();
+    sweep_mixed_kernel<P, D, MODE><<<grid, T, grid_smem<P, MODE>(), s>>>(p);
     return cudaGetLastError();
 }
 
@@ -59,10 +65,10 @@ cudaError_t sweep_launch_mixed(int P, int mode, const SweepParams& p, dim3 grid,
 
 template <int P, int MODE> static cudaError_t attr_d() {
     cudaError_t e = cudaSuccess;
-    const int b = (int)SweepSmem<float, P, MODE>::bytes();
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 0, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    const int g = (int)grid_smem<P, MODE>(), b = (int)SweepSmem<float, P, MODE>::bytes();
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 0, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, g);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, g);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, g);
     if constexpr (P >= 16) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 0, MODE, KIND_AMR>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(sweep_mixed_kernel<P, 1, MODE, KIND_AMR>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
@@ -148,8 +154,8 @@ int sweep_tma_ctas_per_sm_mixed() {
 // resident CTAs per SM of the uniform-grid sweep (the three axes share registers and shared memory)
 template <int P, int MODE> static int occupancy() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_mixed_kernel<P, 0, MODE>, SWEEP_THREADS,
-                                                      SweepSmem<float, P, MODE>::bytes()) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_mixed_kernel<P, 0, MODE>, sweep_threads<float, MODE, KIND_GRID>(),
+                                                      grid_smem<P, MODE>()) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }

@@ -441,6 +441,14 @@ static bool sweep_grid_too_large(const emg_uniform* h, int d) {
     return h->sweepGrid[d].y > 65535u || h->mesh.n[h->other_axis[d]] > 65535;
 }
 
+// threads per CTA of the uniform-grid sweep of the handle's form and mode
+static int sweep_cta_threads(const emg_uniform* h) {
+    if (h->opts.mode != EMG_MODE_WENO) return SWEEP_THREADS;
+    return h->opts.precision == EMG_PRECISION_MIXED      ? sweep_threads<float, MODE_WENO, KIND_GRID>()
+           : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_threads<F64Fast, MODE_WENO, KIND_GRID>()
+                                                         : sweep_threads<double, MODE_WENO, KIND_GRID>();
+}
+
 // Segment length of the sweep along d: the fewest (waves of CTAs) × (rows a
 // CTA streams, seg + 6 with the halo) over the slots of resident CTAs of the
 // whole GPU; a shorter segment only when it is 5 % cheaper. Short segments
@@ -453,11 +461,11 @@ int64_t plan_seg(const emg_uniform* h, int d, int P) {
         cudaGetLastError();
         sms = 148;
     }
-    // at most 3 resident CTAs per SM count as slots: a fourth shares the SM's
+    // at most 3 resident CTAs of 256 threads per SM count as slots: a fourth shares the SM's
     // FP64 pipe instead of adding throughput, so cutting pencils into shorter
     // segments to fill it only adds halo rows (the 2-D 512² step measured
     // 20 % slower planned for 4)
-    const int per_sm = std::min(3, h->opts.precision == EMG_PRECISION_MIXED      ? sweep_ctas_per_sm_mixed(P, h->opts.mode)
+    const int per_sm = std::min(3 * SWEEP_THREADS / sweep_cta_threads(h), h->opts.precision == EMG_PRECISION_MIXED      ? sweep_ctas_per_sm_mixed(P, h->opts.mode)
                                    : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_ctas_per_sm_fast(P, h->opts.mode)
                                                                                  : sweep_ctas_per_sm_f64(P, h->opts.mode));
     const int64_t slots = (int64_t)sms * per_sm;
@@ -494,8 +502,9 @@ void plan_sweeps(emg_uniform* h) {
         h->lane_axis[d] = lane;
         h->other_axis[d] = other;
         const int64_t pencils = h->mesh.n[lane] * h->mesh.n[other];
-        // hybrid rings hold RM + 9 rows: P = 16 keeps them at 2 CTAs per SM
-        int P = h->opts.mode == EMG_MODE_HYBRID ? 16 : 32;
+        // hybrid rings hold RM + 9 rows: P = 16 keeps them at 2 CTAs per SM; CTAs
+        // of 128 threads stream 8 rows of 16 pencils a round
+        int P = h->opts.mode == EMG_MODE_HYBRID || sweep_cta_threads(h) == 128 ? 16 : 32;
         if (pencils <= 8)
             P = 8;
         else if (pencils <= 16)
@@ -605,6 +614,13 @@ void setup_tma(emg_uniform* h) {
             if (r != CUDA_SUCCESS) return;
         }
     h->tma = 1;
+    // the staged sweeps take 32 pencils per CTA whatever the form's plain loads take
+    for (int d = 0; d < 3; d++)
+        if (h->active[d] && h->sweepP[d] == 16 && h->mesh.n[h->lane_axis[d]] > 16) {
+            h->sweepP[d] = 32;
+            h->sweepSeg[d] = (int)plan_seg(h, d, 32);
+            h->sweepGrid[d] = sweep_grid(h, d, 32, h->sweepSeg[d]);
+        }
 }
 
 int launch_stage(emg_uniform* h, int stage) {
