@@ -15,6 +15,7 @@
 #include "uniform_internal.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -449,41 +450,59 @@ static int sweep_cta_threads(const emg_uniform* h) {
                                                          : sweep_threads<double, MODE_WENO, KIND_GRID>();
 }
 
-// Segment length of the sweep along d: the fewest (waves of CTAs) × (rows a
-// CTA streams, seg + 6 with the halo) over the slots of resident CTAs of the
-// whole GPU; a shorter segment only when it is 5 % cheaper. Short segments
-// fill the SMs on small grids, and a wave count just above a whole number is
-// avoided.
-int64_t plan_seg(const emg_uniform* h, int d, int P) {
+// Cost of sweeping along d with P pencils per CTA and segments of `seg` cells,
+// in rounds of a CTA that has its SM to itself. A CTA computes RM = threads/P
+// midpoints of every pencil per round and seg + 5 of them in all; a round takes
+// longer the more warps share the SM's FP64 pipe (a 256-thread CTA alone about
+// 9 µs in the plain form, three of them 13.6 µs: 256³, 33 rounds); beyond 24
+// warps CTAs wait for a slot.
+static double sweep_cost(const emg_uniform* h, int d, int P, int64_t seg, int sms, int per_sm) {
     const int64_t nd = h->mesh.n[d], pencils = h->mesh.n[h->lane_axis[d]] * h->mesh.n[h->other_axis[d]];
+    const int T = sweep_cta_threads(h), RM = T / P;
+    const int64_t ctas = (pencils + P - 1) / P * ((nd + seg - 1) / seg), slots = (int64_t)sms * per_sm;
+    const double rounds = (double)((seg + 5 + RM - 1) / RM);
+    auto shared = [&](int64_t k) { return 1.0 + 0.25 * std::max<double>(0.0, (double)k * T / SWEEP_THREADS - 1.0); };
+    const int64_t rest = ctas % slots;
+    return rounds * ((double)(ctas / slots) * shared(per_sm) + (rest ? shared((rest + sms - 1) / sms) : 0.0));
+}
+
+// Segment length of the sweep along d with P pencils per CTA, and its cost:
+// short segments fill the SMs on small grids, long ones save halo rows; a
+// shorter segment is taken only when it is 5 % cheaper.
+int64_t plan_seg(const emg_uniform* h, int d, int P, double* cost_out) {
+    const int64_t nd = h->mesh.n[d];
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         cudaGetLastError();
         sms = 148;
     }
-    // at most 3 resident CTAs of 256 threads per SM count as slots: a fourth shares the SM's
-    // FP64 pipe instead of adding throughput, so cutting pencils into shorter
-    // segments to fill it only adds halo rows (the 2-D 512² step measured
-    // 20 % slower planned for 4)
-    const int per_sm = std::min(3 * SWEEP_THREADS / sweep_cta_threads(h), h->opts.precision == EMG_PRECISION_MIXED      ? sweep_ctas_per_sm_mixed(P, h->opts.mode)
-                                   : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_ctas_per_sm_fast(P, h->opts.mode)
-                                                                                 : sweep_ctas_per_sm_f64(P, h->opts.mode));
-    const int64_t slots = (int64_t)sms * per_sm;
-    const int64_t tiles = (pencils + P - 1) / P;
+    // at most 3 resident CTAs of 256 threads per SM count as slots: a fourth shares
+    // the SM's FP64 pipe instead of adding throughput, so cutting pencils into
+    // shorter segments to fill it only adds halo rows
+    // (the kernels and the devices are the same for every handle: asked once)
+    static std::atomic<int> known[3][3][3];
+    std::atomic<int>& slot = known[h->opts.precision][h->opts.mode][P == 8 ? 0 : (P == 16 ? 1 : 2)];
+    int resident = slot.load(std::memory_order_relaxed);
+    if (!resident) {
+        resident = h->opts.precision == EMG_PRECISION_MIXED      ? sweep_ctas_per_sm_mixed(P, h->opts.mode)
+                   : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_ctas_per_sm_fast(P, h->opts.mode)
+                                                                 : sweep_ctas_per_sm_f64(P, h->opts.mode);
+        slot.store(resident, std::memory_order_relaxed);
+    }
+    const int per_sm = std::min(3 * SWEEP_THREADS / sweep_cta_threads(h), resident);
     int64_t best = nd;
     double best_cost = 1e300;
-    for (int64_t k = 1; k <= nd; k++) {
+    for (int64_t k = 1; k <= nd && k <= 65535; k++) {
         const int64_t seg = (nd + k - 1) / k;
         if (k > 1 && seg < 16) break;
         if ((nd + seg - 1) / seg != k) continue;  // same seg as a smaller k
-        const int64_t ctas = tiles * k;
-        if (k > 65535) break;
-        const double cost = (double)((ctas + slots - 1) / slots) * (double)(seg + 6);
-        if (cost < best_cost * 0.95) {  // shorter segments only for a clear gain
+        const double cost = sweep_cost(h, d, P, seg, sms, per_sm);
+        if (cost < best_cost * 0.95) {
             best_cost = cost;
             best = seg;
         }
     }
+    if (cost_out) *cost_out = best_cost;
     return best;
 }
 
@@ -502,14 +521,24 @@ void plan_sweeps(emg_uniform* h) {
         h->lane_axis[d] = lane;
         h->other_axis[d] = other;
         const int64_t pencils = h->mesh.n[lane] * h->mesh.n[other];
-        // hybrid rings hold RM + 9 rows: P = 16 keeps them at 2 CTAs per SM; CTAs
-        // of 128 threads stream 8 rows of 16 pencils a round
+        // Pencils per CTA: 32 on large grids (16 for the hybrid rings, which hold
+        // RM + 9 rows, and for CTAs of 128 threads: 8 rows a round). Fewer pencils
+        // make taller rounds: a grid too small to fill the SMs then runs its
+        // segments in one round instead of three (192², 24-cell segments: 8
+        // pencils × 32 rows on 192 CTAs), at the price of shorter row reads.
         int P = h->opts.mode == EMG_MODE_HYBRID || sweep_cta_threads(h) == 128 ? 16 : 32;
-        if (pencils <= 8)
-            P = 8;
-        else if (pencils <= 16)
-            P = 16;
-        const int64_t seg = plan_seg(h, d, P);
+        while (P > 8 && pencils <= P / 2) P /= 2;
+        double cost = 0.0;
+        int64_t seg = plan_seg(h, d, P, &cost);
+        for (int Q = P / 2; Q >= 8; Q /= 2) {
+            double c = 0.0;
+            const int64_t s2 = plan_seg(h, d, Q, &c);
+            if (c < 0.9 * cost) {
+                P = Q;
+                seg = s2;
+                cost = c;
+            }
+        }
         h->sweepP[d] = P;
         h->sweepSeg[d] = (int)seg;
         h->sweepGrid[d] = sweep_grid(h, d, P, seg);
@@ -616,9 +645,9 @@ void setup_tma(emg_uniform* h) {
     h->tma = 1;
     // the staged sweeps take 32 pencils per CTA whatever the form's plain loads take
     for (int d = 0; d < 3; d++)
-        if (h->active[d] && h->sweepP[d] == 16 && h->mesh.n[h->lane_axis[d]] > 16) {
+        if (h->active[d] && h->sweepP[d] < 32 && h->mesh.n[h->lane_axis[d]] > 16) {
             h->sweepP[d] = 32;
-            h->sweepSeg[d] = (int)plan_seg(h, d, 32);
+            h->sweepSeg[d] = (int)plan_seg(h, d, 32, nullptr);
             h->sweepGrid[d] = sweep_grid(h, d, 32, h->sweepSeg[d]);
         }
 }
@@ -768,7 +797,7 @@ int autotune_sweeps(emg_uniform* h) {
         for (int P : {8, 16, 32}) {
             if (P > 8 && pencils <= P / 2) continue;                         // lanes mostly idle
             if (P == 32 && h->opts.mode == EMG_MODE_HYBRID) continue;  // hybrid rings: one CTA per SM at P = 32
-            const int64_t planned = plan_seg(h, d, P);
+            const int64_t planned = plan_seg(h, d, P, nullptr);
             std::set<int64_t> segs = {nd, (nd + 1) / 2, (nd + 3) / 4, planned, std::min(nd, 2 * planned), (planned + 1) / 2};
             for (int64_t seg : segs) {
                 if (seg < 16 && seg != nd) continue;
