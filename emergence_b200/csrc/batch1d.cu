@@ -60,6 +60,8 @@ struct Inst {
 // Ghost layers of every instance (C/solver.rs:278-348 on a 1-D mesh).
 __global__ void batch_ghosts(double* u, int64_t ntot, Inst* inst, int ninst, int kind_lo, int kind_hi, EosD eos,
                              const double* st_lo, const double* st_hi) {
+    dependency_wait();
+    dependents_may_start();
     const int i = blockIdx.x;
     if (i >= ninst || inst[i].done) return;
     const int64_t off = inst[i].off, n = inst[i].n;
@@ -93,6 +95,8 @@ __global__ void batch_ghosts(double* u, int64_t ntot, Inst* inst, int ninst, int
 // CFL rate of each instance and its dt (C/solver.rs:478-523, :758-768)
 __global__ void batch_begin(const double* __restrict__ u, int64_t ntot, Inst* inst, double* dtv, int ninst, double cfl,
                             double t_end, EosD eosd) {
+    dependency_wait();
+    dependents_may_start();
     const int i = blockIdx.x;
     if (i >= ninst) return;
     Inst& I = inst[i];
@@ -135,6 +139,8 @@ __global__ void batch_begin(const double* __restrict__ u, int64_t ntot, Inst* in
 }
 
 __global__ void batch_end(Inst* inst, int ninst, int* active) {
+    dependency_wait();
+    dependents_may_start();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ninst) return;
     Inst& I = inst[i];
@@ -396,9 +402,8 @@ struct emg_batch1d {
 
     int stage(int s) {
         double* in = s == 1 ? u : (s == 2 ? sa : sb);
-        batch_ghosts<<<ninst, 32, 0, stream>>>(in, ntot, inst, ninst, bc[0].kind, bc[1].kind,
-                                                EosD{eos.gamma, eos.p_inf, eos.b, eos.q}, dstate, dstate + 5);
-        B_CUDA(cudaGetLastError());
+        B_CUDA(launch_dependent(batch_ghosts, ninst, 32, 0, stream, in, ntot, inst, ninst, bc[0].kind, bc[1].kind,
+                                EosD{eos.gamma, eos.p_inf, eos.b, eos.q}, dstate, dstate + 5));
         SweepParams p{};
         p.uin = in;
         p.ctl = ctl;
@@ -662,12 +667,13 @@ int emg_batch1d_run_to(emg_batch1d* h, double t_end, uint64_t* launched) {
     for (;;) {
         // a batch of steps between checks on the host
         for (int k = 0; k < 16; k++) {
-            batch_begin<<<h->ninst, 256, 0, h->stream>>>(h->u, h->ntot, h->inst, h->dtv, h->ninst, h->opts.cfl, t_end, e);
+            B_CUDA(launch_dependent(batch_begin, h->ninst, 256, 0, h->stream, h->u, h->ntot, h->inst, h->dtv, h->ninst,
+                                    h->opts.cfl, t_end, e));
             for (int s = 1; s <= 3; s++) {
                 int rc = h->stage(s);
                 if (rc) return rc;
             }
-            batch_end<<<(h->ninst + 255) / 256, 256, 0, h->stream>>>(h->inst, h->ninst, h->active);
+            B_CUDA(launch_dependent(batch_end, (h->ninst + 255) / 256, 256, 0, h->stream, h->inst, h->ninst, h->active));
             B_CUDA(cudaGetLastError());
         }
         issued += 16;
@@ -775,12 +781,13 @@ int emg_batch1d_record(emg_batch1d* h, double t_end, uint64_t checkpoint_every, 
                 }
                 B_CUDA(cudaMemcpyAsync(h->ckpt[b / K], h->u, h->state_bytes(), cudaMemcpyDeviceToDevice, h->stream));
             }
-            batch_begin<<<h->ninst, 256, 0, h->stream>>>(h->u, h->ntot, h->inst, h->dtv, h->ninst, h->opts.cfl, t_end, e);
+            B_CUDA(launch_dependent(batch_begin, h->ninst, 256, 0, h->stream, h->u, h->ntot, h->inst, h->dtv, h->ninst,
+                                    h->opts.cfl, t_end, e));
             B_CUDA(cudaMemcpyAsync(h->rec_dt + b * h->ninst, h->dtv, h->ninst * sizeof(double), cudaMemcpyDeviceToDevice,
                                    h->stream));
             for (int st = 1; st <= 3; st++)
                 if ((rc = h->stage(st))) return rc;
-            batch_end<<<(h->ninst + 255) / 256, 256, 0, h->stream>>>(h->inst, h->ninst, h->active);
+            B_CUDA(launch_dependent(batch_end, (h->ninst + 255) / 256, 256, 0, h->stream, h->inst, h->ninst, h->active));
             B_CUDA(cudaGetLastError());
         }
         int act = 0;

@@ -46,6 +46,8 @@ struct FiveGhostParams {
 // Ghost layers along d for every (a, b) of the other padded axes
 // (solver.rs:278-348, boundary.rs:34-96); reflecting axes have n >= ng.
 __global__ void five_ghost_kernel(const FiveGhostParams p) {
+    dependency_wait();
+    dependents_may_start();
     if (p.ctl->done) return;
     const Five s = Five::from(p.sys);
     const int64_t total = p.m[p.e0] * p.m[p.e1] * p.ng;
@@ -251,13 +253,9 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) five_sweep_kernel(const Five
 
 template <int P, int MODE> cudaError_t five_launch_d(const FiveSweepParams& p, dim3 grid, cudaStream_t s) {
     const size_t b = FiveSmem<P, MODE>::bytes();
-    if (p.d == 0)
-        five_sweep_kernel<P, 0, MODE><<<grid, SWEEP_THREADS, b, s>>>(p);
-    else if (p.d == 1)
-        five_sweep_kernel<P, 1, MODE><<<grid, SWEEP_THREADS, b, s>>>(p);
-    else
-        five_sweep_kernel<P, 2, MODE><<<grid, SWEEP_THREADS, b, s>>>(p);
-    return cudaGetLastError();
+    if (p.d == 0) return launch_dependent(five_sweep_kernel<P, 0, MODE>, grid, SWEEP_THREADS, b, s, p);
+    if (p.d == 1) return launch_dependent(five_sweep_kernel<P, 1, MODE>, grid, SWEEP_THREADS, b, s, p);
+    return launch_dependent(five_sweep_kernel<P, 2, MODE>, grid, SWEEP_THREADS, b, s, p);
 }
 template <int MODE> cudaError_t five_launch_p(int P, const FiveSweepParams& p, dim3 grid, cudaStream_t s) {
     switch (P) {
@@ -449,9 +447,8 @@ struct emg_five {
             }
             p.sys = sys;
             const int64_t work = m[p.e0] * m[p.e1] * p.ng;
-            five_ghost_kernel<<<kernel_grid(work, 256), 256, 0, stream>>>(p);
+            EMG_CUDA(launch_dependent(five_ghost_kernel, kernel_grid(work, 256), 256, 0, stream, p));
             launches++;
-            EMG_CUDA(cudaGetLastError());
         }
         return EMG_OK;
     }

@@ -366,6 +366,8 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
         __shared__ unsigned int s_fallback, s_limited, s_weno;
         __shared__ int64_t s_loff[P];
         __shared__ int s_lok[P];
+        dependency_wait();
+        dependents_may_start();
         if (p.ctl->done) return;
         const double dt = p.ctl->dt;
         const int tid = threadIdx.x;

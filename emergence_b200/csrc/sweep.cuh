@@ -28,6 +28,7 @@
 // combines midpoints f..f+4; cell c (0..Ls−1) is row c+5 and reads faces c
 // and c+1.
 #pragma once
+#include "launch.cuh"
 #include "physics.cuh"
 #include "quotient.cuh"
 #include "tma.cuh"
@@ -654,6 +655,8 @@ struct Sweep {
         __shared__ unsigned int s_fallback, s_limited, s_weno;
         __shared__ double s_rate[T / 32];
 
+        dependency_wait();
+        dependents_may_start();
         const StepCtl* ctl = p.ctl;
         if (ctl->done) return;
         const double dt = ctl->dt;

@@ -30,8 +30,7 @@ cudaError_t sweep_launch_amr_f64(int P, int mode, const SweepParams& p, dim3 gri
 }
 
 template <int P, int D, int MODE> static cudaError_t launch(const SweepParams& p, dim3 grid, cudaStream_t s) {
-    sweep_f64_kernel<P, D, MODE><<<grid, SWEEP_THREADS, SweepSmem<double, P, MODE>::bytes(), s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(sweep_f64_kernel<P, D, MODE, KIND_GRID>, grid, SWEEP_THREADS, SweepSmem<double, P, MODE>::bytes(), s, p);
 }
 
 template <int P, int MODE> static cudaError_t launch_d(const SweepParams& p, dim3 grid, cudaStream_t s) {
@@ -79,8 +78,7 @@ template <int MODE> static cudaError_t attr_p() {
 
 // batched independent 1-D lines along axis 0, P = 32 segments per CTA
 template <int MODE> static cudaError_t launch_batch(const SweepParams& p, dim3 grid, cudaStream_t s) {
-    sweep_f64_kernel<32, 0, MODE, KIND_BATCH><<<grid, SWEEP_THREADS, SweepSmem<double, 32, MODE>::bytes(), s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(sweep_f64_kernel<32, 0, MODE, KIND_BATCH>, grid, SWEEP_THREADS, SweepSmem<double, 32, MODE>::bytes(), s, p);
 }
 cudaError_t sweep_launch_batch_f64(int mode, const SweepParams& p, dim3 grid, cudaStream_t s) {
     switch (mode) {

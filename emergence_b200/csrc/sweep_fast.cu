@@ -31,8 +31,7 @@ template <int MODE> static cudaError_t launch_amr_p(int P, const SweepParams& p,
 }
 // batched independent 1-D lines along axis 0, P = 32 segments per CTA
 template <int MODE> static cudaError_t launch_batch(const SweepParams& p, dim3 grid, cudaStream_t s) {
-    sweep_fast_kernel<32, 0, MODE, KIND_BATCH><<<grid, SWEEP_THREADS, SweepSmem<F64Fast, 32, MODE>::bytes(), s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(sweep_fast_kernel<32, 0, MODE, KIND_BATCH>, grid, SWEEP_THREADS, SweepSmem<F64Fast, 32, MODE>::bytes(), s, p);
 }
 cudaError_t sweep_launch_batch_fast(int mode, const SweepParams& p, dim3 grid, cudaStream_t s) {
     switch (mode) {
@@ -54,8 +53,7 @@ cudaError_t sweep_launch_amr_fast(int P, int mode, const SweepParams& p, dim3 gr
 
 template <int P, int D, int MODE> static cudaError_t launch(const SweepParams& p, dim3 grid, cudaStream_t s) {
     constexpr int T = sweep_threads<F64Fast, MODE, KIND_GRID>();
-    sweep_fast_kernel<P, D, MODE><<<grid, T, grid_smem<P, MODE>(), s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(sweep_fast_kernel<P, D, MODE, KIND_GRID>, grid, T, grid_smem<P, MODE>(), s, p);
 }
 
 template <int P, int MODE> static cudaError_t launch_d(const SweepParams& p, dim3 grid, cudaStream_t s) {

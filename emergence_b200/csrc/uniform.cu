@@ -119,6 +119,8 @@ struct CharStencilD {
 // (C/solver.rs:278-348; G/kernels.cu:567-614). Only interior cells along d
 // are read, so threads are independent.
 __global__ void ghost_kernel(const GhostParams p) {
+    dependency_wait();
+    dependents_may_start();
     if (p.ctl->done) return;
     const Eos<double> e = Eos<double>::from(p.eos);
     const int64_t total = p.m[p.e0] * p.m[p.e1] * p.ng;
@@ -272,6 +274,8 @@ __global__ void ctl_reset_rate(StepCtl* ctl) {
 
 // Host-given dt (Solver::step / GpuSolver::step).
 __global__ void ctl_begin_host(StepCtl* ctl, double dt) {
+    dependency_wait();
+    dependents_may_start();
     ctl->dt = dt;
     ctl->done = 0;
     ctl->status = 0;
@@ -280,7 +284,7 @@ __global__ void ctl_begin_host(StepCtl* ctl, double dt) {
 
 // Device dt = min(cfl / rate, t_end − t) with the stopping rule and collapse
 // check of Solver::run_to (C/solver.rs:758-768).
-__global__ void ctl_begin_device(StepCtl* ctl, double cfl) {
+__device__ __forceinline__ static void begin_step(StepCtl* ctl, double cfl) {
     if (ctl->done) return;
     if (ctl->status) {  // the previous step left an inadmissible state
         ctl->done = 1;
@@ -310,6 +314,28 @@ __global__ void ctl_begin_device(StepCtl* ctl, double cfl) {
     ctl->dt = dt;
     ctl->rate_bits = 0ull;
 }
+__device__ __forceinline__ static void end_step(StepCtl* ctl) {
+    if (ctl->done) return;
+    ctl->t = ctl->t + ctl->dt;
+    ctl->steps += 1;
+}
+__global__ void ctl_begin_device(StepCtl* ctl, double cfl) {
+    dependency_wait();
+    dependents_may_start();
+    begin_step(ctl, cfl);
+}
+__global__ void ctl_end(StepCtl* ctl) {
+    dependency_wait();
+    dependents_may_start();
+    end_step(ctl);
+}
+// the end of one step and the begin of the next, between the steps of a run
+__global__ void ctl_next(StepCtl* ctl, double cfl) {
+    dependency_wait();
+    dependents_may_start();
+    end_step(ctl);
+    begin_step(ctl, cfl);
+}
 
 // Fixed scratch of the allocation-free step: a 256-byte control block, then
 // the two stage buffers and the residual for grids up to
@@ -327,12 +353,6 @@ __global__ void ctl_reset_all(StepCtl* ctl, double dt) {
         ctl->dt = dt;
         ctl->t_end = INFINITY;
     }
-}
-
-__global__ void ctl_end(StepCtl* ctl) {
-    if (ctl->done) return;
-    ctl->t = ctl->t + ctl->dt;
-    ctl->steps += 1;
 }
 
 // Σ u·vol over interior cells: per-block partial sums, then one block adds
@@ -569,8 +589,7 @@ int launch_ghosts(emg_uniform* h, double* arr) {
         p.eos = EosD{h->eos.gamma, h->eos.p_inf, h->eos.b, h->eos.q};
         const int64_t work = h->m[p.e0] * h->m[p.e1] * p.ng;
         ProfScope ps(h, EMG_K_GHOST);
-        ghost_kernel<<<kernel_grid(work, 256), 256, 0, h->stream>>>(p);
-        EMG_CUDA(cudaGetLastError());
+        EMG_CUDA(launch_dependent(ghost_kernel, kernel_grid(work, 256), 256, 0, h->stream, p));
     }
     return EMG_OK;
 }
@@ -838,15 +857,15 @@ int autotune_sweeps(emg_uniform* h) {
     return EMG_OK;
 }
 
-int launch_step_body(emg_uniform* h) {
+int launch_step_body(emg_uniform* h, bool next) {
     for (int s = 1; s <= 3; s++) {
         int rc = launch_stage(h, s);
         if (rc) return rc;
     }
     {
         ProfScope ps(h, EMG_K_CFL);
-        ctl_end<<<1, 1, 0, h->stream>>>(h->ctl);
-        EMG_CUDA(cudaGetLastError());
+        EMG_CUDA(next ? launch_dependent(ctl_next, 1, 1, 0, h->stream, h->ctl, h->opts.cfl)
+                      : launch_dependent(ctl_end, 1, 1, 0, h->stream, h->ctl));
     }
     // host-side face statistics (every face of every pencil, each stage)
     uint64_t f = 0;
@@ -1226,11 +1245,12 @@ int emg_uniform_advance(emg_uniform* h, uint64_t nsteps, double t_end, uint64_t*
     uint64_t issued = 0;
     while (issued < nsteps) {
         const uint64_t batch = bounded ? std::min<uint64_t>(nsteps - issued, 8) : nsteps - issued;
-        for (uint64_t s = 0; s < batch; s++) {
-            ctl_begin_device<<<1, 1, 0, h->stream>>>(h->ctl, h->opts.cfl);
-            EMG_CUDA(cudaGetLastError());
+        if (batch > 0) {
+            EMG_CUDA(launch_dependent(ctl_begin_device, 1, 1, 0, h->stream, h->ctl, h->opts.cfl));
             h->launches++;
-            rc = launch_step_body(h);
+        }
+        for (uint64_t s = 0; s < batch; s++) {
+            rc = launch_step_body(h, s + 1 < batch);
             if (rc) return rc;
         }
         issued += batch;

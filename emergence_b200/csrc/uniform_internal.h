@@ -89,8 +89,9 @@ struct emg_uniform {
 namespace emg {
 // ghost fill of `arr` (padded SoA) along every active axis, in axis order
 int launch_ghosts(emg_uniform* h, double* arr);
-// three SSP-RK3 stages and the time advance of one step (dt read from the control block)
-int launch_step_body(emg_uniform* h);
+// three SSP-RK3 stages and the time advance of one step (dt read from the control
+// block); `next`: the device also forms the time step of the one that follows
+int launch_step_body(emg_uniform* h, bool next = false);
 // CFL rate of the current state into the control block, if not already there
 int ensure_rate(emg_uniform* h);
 // control block → host mirror (synchronizes the stream)
