@@ -789,6 +789,52 @@ struct emg_amr {
         off.push_back((int)slot.size());
     }
 
+    // Cuts the chains along d where that makes their sweep shorter. A CTA runs
+    // one round of RM = 256/P rows after another over its chain, so on a small
+    // hierarchy (2-D, 1600 leaves: 165 chain CTAs for 444 places) 8-block chains
+    // leave SMs idle; on a large one shorter chains only add the 5 rows each
+    // recomputes at its end. The cost is that of the uniform sweep's planner: a
+    // round takes 1 + ¼(k − 1) of its time alone with k CTAs on the SM, at most
+    // 3. Results do not depend on the cut (the blocks beside it exchange their
+    // values through the ghost copies again).
+    void shorten_chains(int d, std::vector<int>& off) const {
+        int o[2], no = 0;
+        for (int e = 0; e < 3; e++)
+            if (e != d) o[no++] = e;
+        int lane = o[1], other = o[0];
+        if (!act[lane] && act[other]) std::swap(lane, other);
+        const int P = amr_sweep_P(d, lane, other), lw = std::min(P, bd[lane]), RM = SWEEP_THREADS / P;
+        const int64_t groups = (bd[other] + P / lw - 1) / (P / lw), sms = 148, slots = 3 * sms;
+        auto shared = [](int64_t k) { return 1.0 + 0.25 * (double)(k - 1); };
+        int best = AMR_CHAIN_MAX;
+        double best_cost = 1e300;
+        for (int cap = AMR_CHAIN_MAX; cap >= 1; cap /= 2) {
+            // rounds of all CTAs, and of the longest: the waves' total against the critical path
+            int64_t ctas = 0, work = 0, longest = 0;
+            for (size_t c = 0; c + 1 < off.size(); c++)
+                for (int k = off[c]; k < off[c + 1]; k += cap) {
+                    const int64_t r = ((int64_t)std::min(cap, off[c + 1] - k) * bd[d] + 5 + RM - 1) / RM;
+                    ctas += groups;
+                    work += groups * r;
+                    longest = std::max(longest, r);
+                }
+            if (!ctas) return;
+            const double load = (double)work / (double)slots * shared(3);
+            const double path = (double)longest * shared(std::min<int64_t>(3, (ctas + sms - 1) / sms));
+            const double cost = std::max(load, path);
+            if (cost < best_cost * 0.95) {
+                best_cost = cost;
+                best = cap;
+            }
+        }
+        if (best == AMR_CHAIN_MAX) return;
+        std::vector<int> cut;
+        for (size_t c = 0; c + 1 < off.size(); c++)
+            for (int k = off[c]; k < off[c + 1]; k += best) cut.push_back(k);
+        cut.push_back(off.back());
+        off.swap(cut);
+    }
+
     // ---------------------------------------------------------------- layout
     int ensure_layout() {
         if (layout_valid) return upload_map();
@@ -893,6 +939,7 @@ struct emg_amr {
             if (!act[d]) continue;
             std::vector<int> coff, cslot;
             build_chains(d, leaves, coff, cslot);
+            shorten_chains(d, coff);
             for (size_t c = 0; c + 1 < coff.size(); c++)
                 for (int i = coff[c]; i + 1 < coff[c + 1]; i++) next_in_chain[3 * cslot[i] + d] = cslot[i + 1];
             if ((rc = dchain_off[d].put(coff, stream)) || (rc = dchain_slot[d].put(cslot, stream))) return rc;
@@ -1843,6 +1890,7 @@ struct emg_amr {
                 if (!act[d]) continue;
                 std::vector<int> coff, cslot;
                 build_chains(d, ids, coff, cslot, true);
+                shorten_chains(d, coff);
                 if ((rc = L.choff[d].put(coff, stream)) || (rc = L.chslot[d].put(cslot, stream))) return rc;
                 L.nch[d] = (int)coff.size() - 1;
             }
