@@ -12,6 +12,7 @@ Translation units and their FMA policy:
   sweep_mixed.cu  FP32-flux fused sweep                           -fmad=true
   sweep_fast.cu   fast FP64 fused sweep (within 1e-12)            -fmad=true
   five_fast.cu    fast FP64 five-equation sweep                   -fmad=true
+  host_copy.cu    device-to-host copies (no arithmetic)
 The plain FP64 units keep every multiply and add separately rounded so that
 their results round exactly as the reference CPU solver's.
 """
@@ -38,6 +39,7 @@ UNITS = [
     ("sweep_mixed.cu", ["-fmad=true", "-use_fast_math"]),
     ("sweep_fast.cu", ["-fmad=true"]),
     ("five_fast.cu", ["-fmad=true"]),
+    ("host_copy.cu", []),
 ]
 
 

@@ -25,6 +25,7 @@
 #include "uniform_internal.h"
 #include "adjoint.cuh"
 #include "adjoint_launch.h"
+#include "host_copy.h"
 
 #include <cmath>
 #include <cstring>
@@ -724,8 +725,7 @@ int download_aos(emg_adjoint* h, const double* src, double* aos) {
     emg_uniform* f = h->f;
     soa_to_aos<<<grid_for(f->ncell), ADJ_T, 0, f->stream>>>(src, f->staging, f->ncell);
     EMG_CUDA(cudaGetLastError());
-    EMG_CUDA(cudaMemcpyAsync(aos, f->staging, f->ncell * 5 * sizeof(double), cudaMemcpyDeviceToHost, f->stream));
-    EMG_CUDA(cudaStreamSynchronize(f->stream));
+    EMG_CUDA(copy_to_host(aos, f->staging, f->ncell * 5 * sizeof(double), f->stream));
     return EMG_OK;
 }
 

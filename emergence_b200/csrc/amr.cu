@@ -21,6 +21,7 @@
 #include "amr_kernels.cuh"
 #include "amr_regrid.cuh"
 #include "five_launch.h"
+#include "host_copy.h"
 #include "sweep_launch.h"
 
 #include <algorithm>
@@ -35,6 +36,7 @@
 
 namespace emg {
 int set_error(int code, const std::string& msg);
+cudaMemPool_t state_pool(int dev);  // uniform.cu
 }
 
 using namespace emg;
@@ -982,7 +984,7 @@ struct emg_amr {
         AmrDev A = view();
         const int nc = for_sweeps ? ncopy_sweep : ncopy;
         if (nc) {
-            NVK(ghost_copy)<<<nc, COPY_THREADS, 0, stream>>>(A, for_sweeps ? dcopy_sweep.p : dcopy.p);
+            AMR_CUDA(launch_dependent(NVK(ghost_copy), nc, COPY_THREADS, 0, stream, A, for_sweeps ? dcopy_sweep.p : dcopy.p));
             launches++;
         }
         int rc = run_pboxes(dpbox.p, npbox, pbox_max);
@@ -2023,7 +2025,7 @@ struct emg_amr {
         ScLevel& L = sc[l];
         AmrDev A = view();
         if (L.ncopy) {
-            NVK(ghost_copy)<<<L.ncopy, COPY_THREADS, 0, stream>>>(A, L.copies.p);
+            AMR_CUDA(launch_dependent(NVK(ghost_copy), L.ncopy, COPY_THREADS, 0, stream, A, L.copies.p));
             launches++;
         }
         int rc = run_pboxes(L.pboxes.p, L.npbox, L.pmax);
@@ -2683,14 +2685,19 @@ int emg_amr_download(emg_amr* h, double* u, size_t nblocks) {
     if (!u || nblocks < h->blocks.size()) return set_error(EMG_ERR_INVALID, "buffer too small");
     const int nv = h->nv;
     const size_t n = h->blocks.size() * (size_t)h->bcells() * nv;
+    // staging from the library's pool: cudaMalloc and cudaFree of 300 MB stalled
+    // the device for up to some 100 ms per call on a shared host
     double* tmp = nullptr;
-    AMR_CUDA(cudaMalloc(&tmp, n * sizeof(double)));
+    cudaMemPool_t pool = state_pool(h->device);
+    if (!pool) return set_error(EMG_ERR_CUDA, "device memory pool unavailable");
+    AMR_CUDA(cudaMallocFromPoolAsync((void**)&tmp, n * sizeof(double), pool, h->stream));
     AmrDev A = h->view();
     NVK(pool_get_interior)<<<256, 256, 0, h->stream>>>(A, (int)h->blocks.size(), tmp);
-    cudaMemcpyAsync(u, tmp, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    cudaStreamSynchronize(h->stream);
-    cudaFree(tmp);
-    AMR_CUDA(cudaGetLastError());
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = copy_to_host(u, tmp, n * sizeof(double), h->stream);
+    cudaFreeAsync(tmp, h->stream);
+    AMR_CUDA(e);
+    AMR_CUDA(cudaStreamSynchronize(h->stream));
     return EMG_OK;
 }
 

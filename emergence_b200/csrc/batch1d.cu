@@ -15,6 +15,7 @@
 #include "../../include/emergence_b200.h"
 #include "adjoint.cuh"
 #include "adjoint_launch.h"
+#include "host_copy.h"
 #include "sweep_launch.h"
 
 #include <cmath>
@@ -705,8 +706,7 @@ int emg_batch1d_download(emg_batch1d* h, double* u) {
     cudaSetDevice(h->device);
     batch_unpack<<<h->ninst, 256, 0, h->stream>>>(h->u, h->state, h->ntot, h->inst, h->ninst, h->dcoff);
     B_CUDA(cudaGetLastError());
-    B_CUDA(cudaMemcpyAsync(u, h->state, (size_t)h->ncells * 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    B_CUDA(cudaStreamSynchronize(h->stream));
+    B_CUDA(copy_to_host(u, h->state, (size_t)h->ncells * 5 * sizeof(double), h->stream));
     return EMG_OK;
 }
 

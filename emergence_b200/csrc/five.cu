@@ -13,6 +13,7 @@
 // Built with -fmad=false.
 #include "../../include/emergence_b200.h"
 #include "five_launch.h"
+#include "host_copy.h"
 #include "uniform_internal.h"
 
 #include <algorithm>
@@ -744,8 +745,7 @@ int emg_five_download(emg_five* h, double* u_aos, size_t len) {
     if (!u_aos || len != (size_t)h->ncell) return set_error(EMG_ERR_INVALID, "state length does not match the padded mesh");
     five_soa_to_aos<<<kernel_grid(h->ncell, 256), 256, 0, h->stream>>>(h->u, h->staging, h->ncell);
     EMG_CUDA(cudaGetLastError());
-    EMG_CUDA(cudaMemcpyAsync(u_aos, h->staging, (size_t)h->ncell * NF * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    EMG_CUDA(cudaStreamSynchronize(h->stream));
+    EMG_CUDA(copy_to_host(u_aos, h->staging, (size_t)h->ncell * NF * sizeof(double), h->stream));
     return EMG_OK;
 }
 

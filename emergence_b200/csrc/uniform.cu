@@ -12,6 +12,7 @@
 //
 // Built with -fmad=false: the ghost, CFL and control arithmetic must round as
 // the reference CPU solver does.
+#include "host_copy.h"
 #include "uniform_internal.h"
 
 #include <algorithm>
@@ -1018,14 +1019,15 @@ static int check_uniform_args(const emg_mesh* mesh, const emg_bc bc[6], const em
 
 }  // extern "C"
 
-namespace {
-// The large state buffers of uniform-grid solvers come from a library-owned
+namespace emg {
+// The large state buffers of uniform-grid solvers (and the staging of block-AMR
+// downloads) come from a library-owned
 // stream-ordered memory pool per device that keeps up to 32 GB of freed
 // memory: cudaMalloc of a 256^3 state (4 GB over five buffers) costs 5-60 ms,
 // and a solver created after another one was destroyed reuses its memory.
 // emg_release_memory returns the kept memory to the device.
-std::mutex pool_mu;
-cudaMemPool_t pools[64] = {};
+static std::mutex pool_mu;
+static cudaMemPool_t pools[64] = {};
 cudaMemPool_t state_pool(int dev) {
     if (dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(pool_mu);
@@ -1050,6 +1052,7 @@ cudaMemPool_t state_pool(int dev) {
 extern "C" {
 
 int emg_release_memory(void) {
+    release_host_buffer();
     std::lock_guard<std::mutex> lk(pool_mu);
     for (auto& p : pools)
         if (p && cudaMemPoolTrimTo(p, 0) != cudaSuccess) {
@@ -1192,8 +1195,7 @@ int emg_uniform_download(emg_uniform* h, double* u_aos, size_t len) {
     soa_to_aos<<<kernel_grid(h->ncell, 256), 256, 0, h->stream>>>(h->u, h->staging, h->ncell);
     EMG_CUDA(cudaGetLastError());
     h->launches++;
-    EMG_CUDA(cudaMemcpyAsync(u_aos, h->staging, (size_t)h->ncell * 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    EMG_CUDA(cudaStreamSynchronize(h->stream));
+    EMG_CUDA(copy_to_host(u_aos, h->staging, (size_t)h->ncell * 5 * sizeof(double), h->stream));
     return EMG_OK;
 }
 

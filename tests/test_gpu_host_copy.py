@@ -1,0 +1,54 @@
+"""Downloads into pageable memory go through a pinned buffer emptied by several
+host threads above 8 MB (emergence_b200/csrc/host_copy.cu): the same bytes as a
+direct copy into pinned memory, at sizes around the threshold and the 2 MB
+slots, and from two handles at once (needs a B200)."""
+import threading
+
+import numpy as np
+import pytest
+
+from emergence_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(n, seed):
+    from emergence_b200 import GpuSolver
+    s, mesh, u, bc = W.explosion(n, 0.3, seed=seed)
+    return GpuSolver(s, mesh, u, bc=bc), mesh, u
+
+
+@pytest.mark.parametrize("n", [(209690, 1, 1), (209703, 1, 1), (500, 403, 1), (64, 61, 59)])
+def test_pageable_download_equals_the_pinned_one(n):
+    import torch
+    g, mesh, u = _solver(n, 3)
+    pin = torch.empty((mesh.len(), 5), dtype=torch.float64, pin_memory=True).numpy()
+    g.download(out=pin)
+    out = np.full((mesh.len(), 5), np.nan)
+    assert np.array_equal(g.download(out=out), pin)
+    assert np.array_equal(mesh.interior(out), mesh.interior(u))
+
+
+def test_two_handles_download_at_once():
+    pairs = [_solver((64, 64, 64), k) for k in (1, 2)]
+    bad = []
+
+    def run(g, mesh, u):
+        for _ in range(5):
+            if not np.array_equal(mesh.interior(g.download()), mesh.interior(u)):
+                bad.append(1)
+
+    t = [threading.Thread(target=run, args=p) for p in pairs]
+    for x in t:
+        x.start()
+    for x in t:
+        x.join()
+    assert not bad
+
+
+def test_released_buffer_comes_back():
+    from emergence_b200.solver import release_memory
+    g, mesh, u = _solver((64, 64, 64), 5)
+    a = g.download()
+    release_memory()
+    assert np.array_equal(g.download(), a)
