@@ -532,7 +532,7 @@ struct emg_amr {
                 AMR_CUDA(cudaFuncSetAttribute(pbox_fused<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
                 pbox_fused_ready = true;
             }
-            NVK(pbox_fused)<<<nbox, PBOX_THREADS, fused_smem, stream>>>(A, dboxes, (int)maxcells);
+            AMR_CUDA(launch_dependent(NVK(pbox_fused), nbox, PBOX_THREADS, fused_smem, stream, A, dboxes, (int)maxcells));
             launches++;
             AMR_CUDA(cudaGetLastError());
             return EMG_OK;
@@ -640,20 +640,20 @@ struct emg_amr {
         AmrDev A = view();
         const dim3 gr = box_grid(maxcells, nbox);
         // boxes inside the domain: gather and first pass fused, straight into the first pass's output
-        NVK(rbox_gather_pass0)<<<gr, 256, 0, stream>>>(A, dboxes, scr[1], sok[1], rem);
-        NVK(rbox_gather)<<<gr, 256, 0, stream>>>(A, dboxes, scr[0], sok[0], rem, 1);
+        AMR_CUDA(launch_dependent(NVK(rbox_gather_pass0), gr, 256, 0, stream, A, dboxes, scr[1], sok[1], rem));
+        AMR_CUDA(launch_dependent(NVK(rbox_gather), gr, 256, 0, stream, A, dboxes, scr[0], sok[0], rem, 1));
         for (int di = 0; di < (int)dims.size(); di++) {
             if (bsel && !nbsel[di]) continue;
             const dim3 gb(bsel ? (unsigned)nbsel[di] : gr.x, gr.y, 1);
-            NVK(rbox_bc)<<<gb, 256, 0, stream>>>(A, dboxes, scr[0], sok[0], di, bsel ? bsel[di] : nullptr);
+            AMR_CUDA(launch_dependent(NVK(rbox_bc), gb, 256, 0, stream, A, dboxes, scr[0], sok[0], di, bsel ? bsel[di] : nullptr));
             launches++;
         }
         int cur = 0;
         for (int di = 0; di < (int)dims.size(); di++) {
-            NVK(rbox_pass)<<<gr, 256, 0, stream>>>(A, dboxes, scr[cur], sok[cur], scr[1 - cur], sok[1 - cur], di, di == 0 ? 1 : 0);
+            AMR_CUDA(launch_dependent(NVK(rbox_pass), gr, 256, 0, stream, A, dboxes, scr[cur], sok[cur], scr[1 - cur], sok[1 - cur], di, di == 0 ? 1 : 0));
             cur = 1 - cur;
         }
-        NVK(rbox_scatter)<<<gr, 256, 0, stream>>>(A, dboxes, scr[cur]);
+        AMR_CUDA(launch_dependent(NVK(rbox_scatter), gr, 256, 0, stream, A, dboxes, scr[cur]));
         launches += 3 + dims.size();
         AMR_CUDA(cudaGetLastError());
         return EMG_OK;
@@ -991,8 +991,7 @@ struct emg_amr {
         if (rc) return rc;
         if (nbcleaves)
             for (int di = 0; di < (int)dims.size(); di++) {
-                NVK(ghost_bc)<<<box_grid(2 * (int64_t)ng * std::max(bd[0], 1) * std::max(bd[1], 1), nbcleaves), 256, 0, stream>>>(
-                    A, dbcleaves.p, dlevel.p, didx.p, di);
+                AMR_CUDA(launch_dependent(NVK(ghost_bc), box_grid(2 * (int64_t)ng * std::max(bd[0], 1) * std::max(bd[1], 1), nbcleaves), 256, 0, stream, A, dbcleaves.p, dlevel.p, didx.p, di));
                 launches++;
             }
         AMR_CUDA(cudaGetLastError());
@@ -1197,7 +1196,7 @@ struct emg_amr {
             for (int bucket = 0; bucket < 6; bucket++) {
                 const int nf = rface_start[bucket + 1] - rface_start[bucket];
                 if (!nf) continue;
-                NVK(reflux_faces)<<<nf, 256, 0, stream>>>(A, rhs, face, npen, dreflux.p + rface_start[bucket]);
+                AMR_CUDA(launch_dependent(NVK(reflux_faces), nf, 256, 0, stream, A, rhs, face, npen, dreflux.p + rface_start[bucket]));
                 launches++;
             }
             AMR_CUDA(cudaGetLastError());
@@ -1241,8 +1240,7 @@ struct emg_amr {
 
     int rk(int stage) {
         AmrDev A = view();
-        PHK(amr_rk)<<<dim3((unsigned)nleaves, (unsigned)std::min<int64_t>((bcells() + 255) / 256, 16)), 256, 0, stream>>>(
-            A, u0, rhs, dleaves.p, dlevel.p, ddxl.p, stage, ctl, 0);
+        AMR_CUDA(launch_dependent(PHK(amr_rk), dim3((unsigned)nleaves, (unsigned)std::min<int64_t>((bcells() + 255) / 256, 16)), 256, 0, stream, A, u0, rhs, dleaves.p, dlevel.p, ddxl.p, stage, ctl, 0));
         launches++;
         AMR_CUDA(cudaGetLastError());
         record_ev(stage_ev[stage - 1][6]);
@@ -2032,8 +2030,7 @@ struct emg_amr {
         if (rc) return rc;
         if (L.nbcl)
             for (int di = 0; di < (int)dims.size(); di++) {
-                NVK(ghost_bc)<<<box_grid(2 * (int64_t)ng * std::max(bd[0], 1) * std::max(bd[1], 1), L.nbcl), 256, 0, stream>>>(
-                    A, L.bcl.p, dlevel.p, didx.p, di);
+                AMR_CUDA(launch_dependent(NVK(ghost_bc), box_grid(2 * (int64_t)ng * std::max(bd[0], 1) * std::max(bd[1], 1), L.nbcl), 256, 0, stream, A, L.bcl.p, dlevel.p, didx.p, di));
                 launches++;
             }
         AMR_CUDA(cudaGetLastError());
@@ -2091,7 +2088,7 @@ struct emg_amr {
                 NVK(sc_reg_fine)<<<sc[l - 1].face_start[6], 256, 0, stream>>>(A, sc[l - 1].faces.p, face, npen, freg, w, nsub);
                 launches++;
             }
-            PHK(amr_rk)<<<dim3((unsigned)L.nblk, gy), 256, 0, stream>>>(A, u0, rhs, L.blist.p, dlevel.p, ddxl.p, s + 1, ctl, 1);
+            AMR_CUDA(launch_dependent(PHK(amr_rk), dim3((unsigned)L.nblk, gy), 256, 0, stream, A, u0, rhs, L.blist.p, dlevel.p, ddxl.p, s + 1, ctl, 1));
             launches++;
             AMR_CUDA(cudaGetLastError());
         }

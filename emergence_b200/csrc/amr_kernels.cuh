@@ -196,6 +196,8 @@ __global__ void pbox_scatter(const AmrDev A, const PBox* __restrict__ boxes, con
 constexpr int PBOX_THREADS = 512;
 template <int NV>
 __global__ void __launch_bounds__(PBOX_THREADS) pbox_fused(const AmrDev A, const PBox* __restrict__ boxes, int cap) {
+    dependency_wait();
+    dependents_may_start();
     extern __shared__ __align__(16) double pb_smem[];
     double* bufs[2] = {pb_smem, pb_smem + (size_t)cap * NV};
     unsigned char* ok = reinterpret_cast<unsigned char*>(pb_smem + (size_t)2 * cap * NV);
@@ -290,6 +292,8 @@ __global__ void __launch_bounds__(PBOX_THREADS) pbox_fused(const AmrDev A, const
 template <int NV>
 __global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, double* buf, unsigned char* ok,
                             const int* __restrict__ rem, int skip_fast) {
+    dependency_wait();
+    dependents_may_start();
     const RBox b = boxes[blockIdx.x];
     if (skip_fast && b.fast) return;  // gathered inside rbox_gather_pass0
     const int lf = b.l + 1;
@@ -393,6 +397,8 @@ __global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, doub
 template <int NV>
 __global__ void rbox_bc(const AmrDev A, const RBox* __restrict__ boxes, double* buf, unsigned char* ok, int di,
                         const int* __restrict__ sel) {
+    dependency_wait();
+    dependents_may_start();
     const RBox b = boxes[sel ? sel[blockIdx.x] : blockIdx.x];
     const int64_t n = (int64_t)b.sz[0] * b.sz[1] * b.sz[2];
     for (int64_t q = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.y * blockDim.x)
@@ -405,6 +411,8 @@ template <int NV>
 __global__ void __launch_bounds__(256, 4) rbox_pass(const AmrDev A, const RBox* __restrict__ boxes, const double* in,
                                                    const unsigned char* okin,
                           double* outb, unsigned char* okout, int di, int skip_fast) {
+    dependency_wait();
+    dependents_may_start();
     const RBox b = boxes[blockIdx.x];
     if (skip_fast && b.fast) return;  // first pass done by rbox_gather_pass0
     const int d = A.dims[di];
@@ -478,6 +486,8 @@ template <int NV>
 __global__ void __launch_bounds__(256, 4) rbox_gather_pass0(const AmrDev A, const RBox* __restrict__ boxes, double* outb,
                                                            unsigned char* okout,
                                   const int* __restrict__ rem) {
+    dependency_wait();
+    dependents_may_start();
     const RBox b = boxes[blockIdx.x];
     if (!b.fast) return;
     const int lf = b.l + 1;
@@ -595,6 +605,8 @@ __global__ void __launch_bounds__(256, 4) rbox_gather_pass0(const AmrDev A, cons
 // write the restricted box into the ancestor's interior cells [lo, hi)
 template <int NV>
 __global__ void rbox_scatter(const AmrDev A, const RBox* __restrict__ boxes, const double* in) {
+    dependency_wait();
+    dependents_may_start();
     const RBox b = boxes[blockIdx.x];
     int so[3];
     for (int d = 0; d < 3; d++) so[d] = b.hi[d] - b.lo[d];
@@ -621,6 +633,8 @@ struct CopyTask {
 constexpr int COPY_THREADS = 128;
 template <int NV>
 __global__ void __launch_bounds__(COPY_THREADS) ghost_copy(const AmrDev A, const CopyTask* __restrict__ tasks) {
+    dependency_wait();
+    dependents_may_start();
     const CopyTask t = tasks[blockIdx.x];
     int rs[3], sz[3];
     for (int d = 0; d < 3; d++) {
@@ -659,6 +673,8 @@ __global__ void __launch_bounds__(COPY_THREADS) ghost_copy(const AmrDev A, const
 template <int NV>
 __global__ void ghost_bc(const AmrDev A, const int* __restrict__ leaves, const int* __restrict__ level,
                          const int64_t* __restrict__ idx, int di) {
+    dependency_wait();
+    dependents_may_start();
     const int slot = leaves[blockIdx.x];
     const int l = level[slot];
     const int64_t n = (int64_t)A.ext[0] * A.ext[1] * A.ext[2];
@@ -738,6 +754,8 @@ struct RefluxFace {
 template <int NV>
 __global__ void reflux_faces(const AmrDev A, double* rhs, const double* __restrict__ face, int npen,
                              const RefluxFace* __restrict__ tasks) {
+    dependency_wait();
+    dependents_may_start();
     const RefluxFace tk = tasks[blockIdx.x];
     const int d = tk.d;
     const int e0 = d == 0 ? 1 : 0, e1 = d == 2 ? 1 : 2;
@@ -830,6 +848,8 @@ template <class PH>
 __global__ void amr_rk(const AmrDev A, double* u0, const double* __restrict__ rhs, const int* __restrict__ leaves,
                        const int* __restrict__ level, const double* __restrict__ dxl, int stage, StepCtl* ctl,
                        int sc) {
+    dependency_wait();
+    dependents_may_start();
     constexpr int NV = PH::NV;
     const int slot = leaves[blockIdx.x];
     const int l = level[slot];

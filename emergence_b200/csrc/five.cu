@@ -288,13 +288,9 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) five_sweep_amr_kernel(const 
 }
 template <int P, int MODE> cudaError_t five_launch_amr_d(const FiveSweepParams& p, dim3 grid, cudaStream_t s) {
     const size_t b = FiveSmem<P, MODE>::bytes();
-    if (p.d == 0)
-        five_sweep_amr_kernel<P, 0, MODE><<<grid, SWEEP_THREADS, b, s>>>(p);
-    else if (p.d == 1)
-        five_sweep_amr_kernel<P, 1, MODE><<<grid, SWEEP_THREADS, b, s>>>(p);
-    else
-        five_sweep_amr_kernel<P, 2, MODE><<<grid, SWEEP_THREADS, b, s>>>(p);
-    return cudaGetLastError();
+    if (p.d == 0) return launch_dependent(five_sweep_amr_kernel<P, 0, MODE>, grid, SWEEP_THREADS, b, s, p);
+    if (p.d == 1) return launch_dependent(five_sweep_amr_kernel<P, 1, MODE>, grid, SWEEP_THREADS, b, s, p);
+    return launch_dependent(five_sweep_amr_kernel<P, 2, MODE>, grid, SWEEP_THREADS, b, s, p);
 }
 template <int MODE> cudaError_t five_launch_amr_p(int P, const FiveSweepParams& p, dim3 grid, cudaStream_t s) {
     switch (P) {

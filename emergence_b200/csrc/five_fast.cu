@@ -16,13 +16,9 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) five_fast_sweep_kernel(const
 
 template <int P, int MODE, bool AMR> static cudaError_t launch_d(const FiveSweepParams& p, dim3 grid, cudaStream_t s) {
     const size_t b = FiveSmem<P, MODE>::bytes();
-    if (p.d == 0)
-        five_fast_sweep_kernel<P, 0, MODE, AMR><<<grid, SWEEP_THREADS, b, s>>>(p);
-    else if (p.d == 1)
-        five_fast_sweep_kernel<P, 1, MODE, AMR><<<grid, SWEEP_THREADS, b, s>>>(p);
-    else
-        five_fast_sweep_kernel<P, 2, MODE, AMR><<<grid, SWEEP_THREADS, b, s>>>(p);
-    return cudaGetLastError();
+    if (p.d == 0) return launch_dependent(five_fast_sweep_kernel<P, 0, MODE, AMR>, grid, SWEEP_THREADS, b, s, p);
+    if (p.d == 1) return launch_dependent(five_fast_sweep_kernel<P, 1, MODE, AMR>, grid, SWEEP_THREADS, b, s, p);
+    return launch_dependent(five_fast_sweep_kernel<P, 2, MODE, AMR>, grid, SWEEP_THREADS, b, s, p);
 }
 template <int MODE, bool AMR> static cudaError_t launch_p(int P, const FiveSweepParams& p, dim3 grid, cudaStream_t s) {
     switch (P) {

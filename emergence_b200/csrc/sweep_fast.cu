@@ -20,8 +20,7 @@ __global__ void __launch_bounds__(sweep_threads<F64Fast, MODE, KIND>(), sweep_th
 
 // batched block-AMR leaves: P = 16 or 32 pencils, one block per lane set
 template <int P, int D, int MODE> static cudaError_t launch_amr(const SweepParams& p, dim3 grid, cudaStream_t s) {
-    sweep_fast_kernel<P, D, MODE, KIND_AMR><<<grid, SWEEP_THREADS, SweepSmem<F64Fast, P, MODE>::bytes(), s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(sweep_fast_kernel<P, D, MODE, KIND_AMR>, grid, SWEEP_THREADS, SweepSmem<F64Fast, P, MODE>::bytes(), s, p);
 }
 template <int P, int MODE> static cudaError_t launch_amr_d(const SweepParams& p, dim3 grid, cudaStream_t s) {
     return p.d == 0 ? launch_amr<P, 0, MODE>(p, grid, s) : (p.d == 1 ? launch_amr<P, 1, MODE>(p, grid, s) : launch_amr<P, 2, MODE>(p, grid, s));
