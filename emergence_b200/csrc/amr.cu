@@ -638,6 +638,19 @@ struct emg_amr {
                    const int* const* bsel = nullptr, const int* nbsel = nullptr) {
         if (!nbox) return EMG_OK;
         AmrDev A = view();
+        // a patch and, behind the first pass, half of it (each axis of n cells has a
+        // patch of 2n + 8), with a validity byte per cell
+        const size_t fused_smem = (size_t)(maxcells + (maxcells + 1) / 2) * (nv * sizeof(double) + 1);
+        if (fused_smem <= 224 * 1024) {
+            if (!rbox_fused_ready) {
+                AMR_CUDA(cudaFuncSetAttribute(rbox_fused<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+                AMR_CUDA(cudaFuncSetAttribute(rbox_fused<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+                rbox_fused_ready = true;
+            }
+            AMR_CUDA(launch_dependent(NVK(rbox_fused), nbox, RBOX_THREADS, fused_smem, stream, A, dboxes, (int)maxcells, rem));
+            launches++;
+            return EMG_OK;
+        }
         const dim3 gr = box_grid(maxcells, nbox);
         // boxes inside the domain: gather and first pass fused, straight into the first pass's output
         AMR_CUDA(launch_dependent(NVK(rbox_gather_pass0), gr, 256, 0, stream, A, dboxes, scr[1], sok[1], rem));
@@ -976,6 +989,7 @@ struct emg_amr {
         return EMG_OK;
     }
     int64_t pbox_max = 0;
+    bool rbox_fused_ready = false;  // likewise, of rbox_fused
     bool pbox_fused_ready = false;  // dynamic shared-memory opt-in of pbox_fused (per handle and device)
 
     // ghost-extended boxes of every leaf (fill_scratch, C/amr.rs:1113-1221)

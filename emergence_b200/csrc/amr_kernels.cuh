@@ -289,13 +289,11 @@ __global__ void __launch_bounds__(PBOX_THREADS) pbox_fused(const AmrDev A, const
 // (optional) replays a batch of coarsenings in their sequential order: fine
 // block id is absent for box seq when rem[id] < seq, i.e. it was removed by an
 // earlier coarsening of the batch.
+// cells q0, q0 + step, … of a box, at `off` of the buffers; every thread of the
+// CTA takes part
 template <int NV>
-__global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, double* buf, unsigned char* ok,
-                            const int* __restrict__ rem, int skip_fast) {
-    dependency_wait();
-    dependents_may_start();
-    const RBox b = boxes[blockIdx.x];
-    if (skip_fast && b.fast) return;  // gathered inside rbox_gather_pass0
+__device__ __forceinline__ void rbox_gather_cells(const AmrDev& A, const RBox& b, double* buf, unsigned char* ok, int64_t off,
+                                                  const int* __restrict__ rem, int64_t q0, int64_t step) {
     const int lf = b.l + 1;
     const int64_t n = (int64_t)b.sz[0] * b.sz[1] * b.sz[2];
     // fine patch inside the domain spanning at most four blocks per axis: the
@@ -329,7 +327,7 @@ __global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, doub
             s_slot[t] = id;
         }
         __syncthreads();
-        for (int64_t q = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.y * blockDim.x) {
+        for (int64_t q = q0; q < n; q += step) {
             int64_t c[3];
             box_coord(q, b.sz, c);
             int j[3];
@@ -345,17 +343,17 @@ __global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, doub
                 lc[d] = o - j[d] * A.bd[d];
             }
             const int id = s_slot[(j[0] * s_nk[1] + j[1]) * s_nk[2] + j[2]];
-            double* v = buf + (b.off + q) * NV;
+            double* v = buf + (off + q) * NV;
             if (id >= 0) {
                 amr_load<NV>(A, id, amr_cell(A, lc), v);
             } else {
                 for (int k = 0; k < NV; k++) v[k] = 0.0;
             }
-            ok[b.off + q] = id >= 0 ? 1 : 0;
+            ok[off + q] = id >= 0 ? 1 : 0;
         }
         return;
     }
-    for (int64_t q = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.y * blockDim.x) {
+    for (int64_t q = q0; q < n; q += step) {
         int64_t c[3];
         box_coord(q, b.sz, c);
         int64_t gw[3];
@@ -373,7 +371,7 @@ __global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, doub
                 }
             }
         }
-        double* v = buf + (b.off + q) * NV;
+        double* v = buf + (off + q) * NV;
         unsigned char o = 0;
         if (!out) {
             int64_t key[3], lc[3];
@@ -390,8 +388,18 @@ __global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, doub
         }
         if (!o)
             for (int k = 0; k < NV; k++) v[k] = 0.0;
-        ok[b.off + q] = o;
+        ok[off + q] = o;
     }
+}
+template <int NV>
+__global__ void rbox_gather(const AmrDev A, const RBox* __restrict__ boxes, double* buf, unsigned char* ok,
+                            const int* __restrict__ rem, int skip_fast) {
+    dependency_wait();
+    dependents_may_start();
+    const RBox b = boxes[blockIdx.x];
+    if (skip_fast && b.fast) return;  // gathered inside rbox_gather_pass0
+    rbox_gather_cells<NV>(A, b, buf, ok, b.off, rem, blockIdx.y * (int64_t)blockDim.x + threadIdx.x,
+                          (int64_t)gridDim.y * blockDim.x);
 }
 
 template <int NV>
@@ -406,15 +414,11 @@ __global__ void rbox_bc(const AmrDev A, const RBox* __restrict__ boxes, double* 
 }
 
 // one restriction pass along dims[di] with the shifted stencils and the
-// child-average fallback (amr.rs:674-727)
+// child-average fallback (amr.rs:674-727), outputs q0, q0 + step, … of a box
 template <int NV>
-__global__ void __launch_bounds__(256, 4) rbox_pass(const AmrDev A, const RBox* __restrict__ boxes, const double* in,
-                                                   const unsigned char* okin,
-                          double* outb, unsigned char* okout, int di, int skip_fast) {
-    dependency_wait();
-    dependents_may_start();
-    const RBox b = boxes[blockIdx.x];
-    if (skip_fast && b.fast) return;  // first pass done by rbox_gather_pass0
+__device__ __forceinline__ void rbox_pass_cells(const AmrDev& A, const RBox& b, const double* in, const unsigned char* okin,
+                                                double* outb, unsigned char* okout, int64_t off, int di, int64_t q0,
+                                                int64_t step) {
     const int d = A.dims[di];
     int si[3], so[3];
     rbox_size(A, b, di, si);
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(256, 4) rbox_pass(const AmrDev A, const RBox* 
     // stride of d in the box's row-major layout, and its extent
     const int64_t str = d == 0 ? (int64_t)si[1] * si[2] : (d == 1 ? si[2] : 1);
     const int sid = d == 0 ? si[0] : (d == 1 ? si[1] : si[2]);
-    for (int64_t q = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.y * blockDim.x) {
+    for (int64_t q = q0; q < n; q += step) {
         int64_t c[3];
         box_coord(q, so, c);
         const int cd = (int)(d == 0 ? c[0] : (d == 1 ? c[1] : c[2]));
@@ -432,7 +436,7 @@ __global__ void __launch_bounds__(256, 4) rbox_pass(const AmrDev A, const RBox* 
         if (d == 0) c0[0] = 0;
         else if (d == 1) c0[1] = 0;
         else c0[2] = 0;
-        const int64_t row0 = b.off + box_index(c0, si);  // source index at position 0 along d
+        const int64_t row0 = off + box_index(c0, si);  // source index at position 0 along d
         const int base = 2 * cd + 2;
         // positions base − 2 .. base + 7 (every stencil the shifts reach): index
         // and validity, position i = shift + 2 + kk of the unrolled stencils
@@ -471,10 +475,21 @@ __global__ void __launch_bounds__(256, 4) rbox_pass(const AmrDev A, const RBox* 
             for (int k = 0; k < NV; k++) acc[k] = 0.5 * (in[pa * NV + k] + in[pb * NV + k]);
             o = 1;
         }
-        double* ov = outb + (b.off + q) * NV;
+        double* ov = outb + (off + q) * NV;
         for (int k = 0; k < NV; k++) ov[k] = acc[k];
-        okout[b.off + q] = o;
+        okout[off + q] = o;
     }
+}
+template <int NV>
+__global__ void __launch_bounds__(256, 4) rbox_pass(const AmrDev A, const RBox* __restrict__ boxes, const double* in,
+                                                   const unsigned char* okin, double* outb, unsigned char* okout, int di,
+                                                   int skip_fast) {
+    dependency_wait();
+    dependents_may_start();
+    const RBox b = boxes[blockIdx.x];
+    if (skip_fast && b.fast) return;  // first pass done by rbox_gather_pass0
+    rbox_pass_cells<NV>(A, b, in, okin, outb, okout, b.off, di, blockIdx.y * (int64_t)blockDim.x + threadIdx.x,
+                        (int64_t)gridDim.y * blockDim.x);
 }
 
 // Gather and first restriction pass (along dims[0]) in one kernel for boxes
@@ -604,22 +619,63 @@ __global__ void __launch_bounds__(256, 4) rbox_gather_pass0(const AmrDev A, cons
 
 // write the restricted box into the ancestor's interior cells [lo, hi)
 template <int NV>
-__global__ void rbox_scatter(const AmrDev A, const RBox* __restrict__ boxes, const double* in) {
-    dependency_wait();
-    dependents_may_start();
-    const RBox b = boxes[blockIdx.x];
+__device__ __forceinline__ void rbox_scatter_cells(const AmrDev& A, const RBox& b, const double* in, int64_t off, int64_t q0,
+                                                   int64_t step) {
     int so[3];
     for (int d = 0; d < 3; d++) so[d] = b.hi[d] - b.lo[d];
     const int64_t n = (int64_t)so[0] * so[1] * so[2];
     double* u = A.u + (int64_t)b.slot * A.bcell;
-    for (int64_t q = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.y * blockDim.x) {
+    for (int64_t q = q0; q < n; q += step) {
         int64_t c[3];
         box_coord(q, so, c);
         const int64_t ic[3] = {b.lo[0] + c[0], b.lo[1] + c[1], b.lo[2] + c[2]};
         const int64_t cell = amr_cell(A, ic);
-        const double* v = in + (b.off + q) * NV;
+        const double* v = in + (off + q) * NV;
         for (int k = 0; k < NV; k++) u[(int64_t)k * A.ntot + cell] = v[k];
     }
+}
+template <int NV>
+__global__ void rbox_scatter(const AmrDev A, const RBox* __restrict__ boxes, const double* in) {
+    dependency_wait();
+    dependents_may_start();
+    const RBox b = boxes[blockIdx.x];
+    rbox_scatter_cells<NV>(A, b, in, b.off, blockIdx.y * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.y * blockDim.x);
+}
+
+// Whole restriction of a box by one CTA in shared memory, for boxes whose fine
+// patch fits there (2-D blocks of 16²: 40² cells × 5 values, 64 KB, and half as
+// much behind the first pass): gather, boundary passes, one pass per axis,
+// scatter, instead of six to eight launches of a few µs per level of a small
+// hierarchy. `cap` is the largest patch of the launch's boxes.
+constexpr int RBOX_THREADS = 512;
+template <int NV>
+__global__ void __launch_bounds__(RBOX_THREADS, 2) rbox_fused(const AmrDev A, const RBox* __restrict__ boxes, int cap,
+                                                          const int* __restrict__ rem) {
+    dependency_wait();
+    dependents_may_start();
+    extern __shared__ __align__(16) double rb_smem[];
+    const int half = (cap + 1) / 2;
+    double* bufs[2] = {rb_smem, rb_smem + (size_t)cap * NV};
+    unsigned char* oks[2] = {reinterpret_cast<unsigned char*>(bufs[1] + (size_t)half * NV), nullptr};
+    oks[1] = oks[0] + cap;
+    const RBox b = boxes[blockIdx.x];
+    const int64_t q0 = threadIdx.x, step = blockDim.x;
+    rbox_gather_cells<NV>(A, b, bufs[0], oks[0], 0, rem, q0, step);
+    __syncthreads();
+    if (!b.fast) {  // the patch may cross a domain side
+        const int64_t n = (int64_t)b.sz[0] * b.sz[1] * b.sz[2];
+        for (int di = 0; di < A.ndims; di++) {
+            for (int64_t q = q0; q < n; q += step) bc_cell<NV>(A, b.l + 1, b.f0, b.sz, q, di, bufs[0], oks[0], 0);
+            __syncthreads();
+        }
+    }
+    int cur = 0;
+    for (int di = 0; di < A.ndims; di++) {
+        rbox_pass_cells<NV>(A, b, bufs[cur], oks[cur], bufs[1 - cur], oks[1 - cur], 0, di, q0, step);
+        __syncthreads();
+        cur = 1 - cur;
+    }
+    rbox_scatter_cells<NV>(A, b, bufs[cur], 0, q0, step);
 }
 
 // Same-level ghost slab copy (fill_scratch, amr.rs:1176-1187): task =
