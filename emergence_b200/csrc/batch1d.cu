@@ -38,12 +38,13 @@ using namespace emg;
 namespace {
 
 constexpr int NG = 6;
-// cells per segment (one lane of a sweep CTA): short segments keep the CTAs
-// of unfinished instances evenly spread as instances finish at different
-// batch steps (4096 Riemann problems: 24 cells 2.8 s, 32 cells 2.9 s, 64 cells
-// 3.7 s per run, FP64; the 5 halo midpoints per segment cost less than the
-// imbalance of long ones)
-constexpr int SEG = 24;
+// cells per segment (one lane of a sweep CTA). A segment of n cells computes
+// n + 5 midpoints in rounds of 8, so 27 fill four rounds exactly (24 left three
+// of 32 rows idle); short segments keep the CTAs of unfinished instances evenly
+// spread as instances finish at different batch steps (4096 Riemann problems,
+// one frame: 24 cells 32.3 ms, 27 cells 31.1, 35 cells 32.4, 43 cells 33.9, 59
+// cells 36.2).
+constexpr int SEG = 27;
 
 struct Inst {
     int64_t off;   // flat index of the instance's first padded cell
