@@ -1484,9 +1484,10 @@ struct emg_amr {
         if ((rc = grow_det((int64_t)blocks.size()))) return rc;
         AMR_CUDA(cudaMemsetAsync(det, 0, blocks.size() * sizeof(unsigned long long), stream));
         AmrDev A = view();
-        PHK(amr_detail)<<<dim3((unsigned)nleaves, (unsigned)std::min<int64_t>((bcells() + 255) / 256, 16)), 256, 0, stream>>>(
-            A, dleaves.p, det);
-        launches++;
+        const dim3 gd((unsigned)nleaves, (unsigned)std::min<int64_t>((bcells() + 255) / 256, 16));
+        PHK(amr_sensors)<<<gd, 256, 0, stream>>>(A, dleaves.p, rhs);
+        PHK(amr_detail)<<<gd, 256, 0, stream>>>(A, dleaves.p, rhs, det);
+        launches += 2;
         AMR_CUDA(cudaGetLastError());
         std::vector<unsigned long long> bits(blocks.size());
         AMR_CUDA(cudaMemcpyAsync(bits.data(), det, bits.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
@@ -1619,9 +1620,10 @@ struct emg_amr {
         if ((rc = grow_det((int64_t)blocks.size()))) return rc;
         AMR_CUDA(cudaMemsetAsync(det, 0, blocks.size() * sizeof(unsigned long long), stream));
         AmrDev A = view();
-        PHK(amr_detail)<<<dim3((unsigned)nleaves, (unsigned)std::min<int64_t>((bcells() + 255) / 256, 16)), 256, 0, stream>>>(
-            A, dleaves.p, det);
-        launches++;
+        const dim3 gd((unsigned)nleaves, (unsigned)std::min<int64_t>((bcells() + 255) / 256, 16));
+        PHK(amr_sensors)<<<gd, 256, 0, stream>>>(A, dleaves.p, rhs);
+        PHK(amr_detail)<<<gd, 256, 0, stream>>>(A, dleaves.p, rhs, det);
+        launches += 2;
         AMR_CUDA(cudaGetLastError());
         return EMG_OK;
     }

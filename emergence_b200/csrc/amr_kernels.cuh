@@ -1292,41 +1292,65 @@ __global__ void sc_cfl_levels(const AmrDev A, const int* __restrict__ blist, con
     }
 }
 
+// Sensor values of each leaf's interior cells and of the five ghost cells beyond
+// each face, once per cell: `sens` is SoA over the pool's cells (the residual
+// array, which the next stage's first sweep overwrites). Evaluated at every
+// stencil position instead, a cell's two logarithms and its primitive recovery
+// were computed 19 times in 3-D: 2.2 ms for 1590 leaves of 16³.
+template <class PH>
+__global__ void amr_sensors(const AmrDev A, const int* __restrict__ leaves, double* sens) {
+    const int slot = leaves[blockIdx.x];
+    const typename PH::Ctx e = PH::ctx(A);
+    const int b[3] = {A.bd[0], A.bd[1], A.bd[2]};
+    const int n = b[0] * b[1] * b[2];
+    int end[4] = {n, n, n, n};  // interior, then the slabs of each axis
+    for (int d = 0; d < 3; d++) end[d + 1] = end[d] + (A.act[d] ? 10 * (n / b[d]) : 0);
+    for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < end[3]; q += gridDim.y * blockDim.x) {
+        int64_t c[3];
+        if (q < n) {
+            box_coord(q, A.bd, c);
+        } else {
+            const int d = q < end[1] ? 0 : (q < end[2] ? 1 : 2);
+            const int ext[3] = {d == 0 ? 10 : b[0], d == 1 ? 10 : b[1], d == 2 ? 10 : b[2]};
+            int r = q - end[d];
+            c[2] = r % ext[2];
+            r /= ext[2];
+            c[1] = r % ext[1];
+            c[0] = r / ext[1];
+            c[d] = c[d] < 5 ? c[d] - 5 : c[d] - 5 + b[d];
+        }
+        const int64_t cell = (int64_t)slot * A.bcell + amr_cell(A, c);
+        double u[PH::NV], w[PH::NV], sv[PH::NS];
+        for (int k = 0; k < PH::NV; k++) u[k] = A.u[(int64_t)k * A.ntot + cell];
+        PH::prim(e, u, w);
+        PH::sensor(e, w, sv);
+        for (int k = 0; k < PH::NS; k++) sens[(int64_t)k * A.ntot + cell] = sv[k];
+    }
+}
 // Largest relative wavelet detail of each leaf on the system's sensors
 // (block_detail, amr.rs:823-867), over its filled ghost-extended box.
 template <class PH>
-__device__ __forceinline__ void amr_sensor(const AmrDev& A, const typename PH::Ctx& e, const double* u, int64_t cell,
-                                           double* s) {
-    double q[PH::NV], w[PH::NV];
-    for (int k = 0; k < PH::NV; k++) q[k] = u[(int64_t)k * A.ntot + cell];
-    PH::prim(e, q, w);
-    PH::sensor(e, w, s);
-}
-template <class PH>
-__global__ void amr_detail(const AmrDev A, const int* __restrict__ leaves, unsigned long long* det_bits) {
+__global__ void amr_detail(const AmrDev A, const int* __restrict__ leaves, const double* __restrict__ sens,
+                           unsigned long long* det_bits) {
     constexpr int NS = PH::NS;
     const int slot = leaves[blockIdx.x];
     const int64_t n = (int64_t)A.bd[0] * A.bd[1] * A.bd[2];
-    const typename PH::Ctx e = PH::ctx(A);
-    const double* u = A.u + (int64_t)slot * A.bcell;
     const int offs[6] = {-5, -3, -1, 1, 3, 5};
     double mx = 0.0;
     for (int64_t q = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.y * blockDim.x) {
         int64_t c[3];
         box_coord(q, A.bd, c);
-        const int64_t cell = amr_cell(A, c);
+        const int64_t cell = (int64_t)slot * A.bcell + amr_cell(A, c);
         double s0[NS];
-        amr_sensor<PH>(A, e, u, cell, s0);
+        for (int k = 0; k < NS; k++) s0[k] = sens[(int64_t)k * A.ntot + cell];
         for (int i = 0; i < A.ndims; i++) {
             const int d = A.dims[i];
             const int64_t stride = d == 0 ? (int64_t)A.ext[1] * A.ext[2] : (d == 1 ? A.ext[2] : 1);
             double pred[NS];
             for (int k = 0; k < NS; k++) pred[k] = 0.0;
-            for (int m = 0; m < 6; m++) {
-                double sv[NS];
-                amr_sensor<PH>(A, e, u, cell + offs[m] * stride, sv);
-                for (int k = 0; k < NS; k++) pred[k] = pred[k] + A.wr[m] * sv[k];
-            }
+            for (int m = 0; m < 6; m++)
+                for (int k = 0; k < NS; k++)
+                    pred[k] = pred[k] + A.wr[m] * sens[(int64_t)k * A.ntot + cell + offs[m] * stride];
             for (int k = 0; k < NS; k++) {
                 const double dd = fabs(s0[k] - pred[k]);
                 mx = isfinite(dd) ? fmax(mx, dd) : INFINITY;
