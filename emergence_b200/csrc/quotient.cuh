@@ -21,9 +21,12 @@ namespace emg {
 //   result could only be wrong for an a/b that close to a midpoint, and to miss
 //   there takes an error of 1 − 2^-52 ulp, that is a > 2 − 2^-51: no b is above.
 // Operands must stay where nothing over- or underflows and every remainder is
-// exact: denominators in [2^-200, 2^200), numerators zero or in ±[2^-760,
-// 2^760). Violations are collected in `bad`, and the caller then evaluates the
-// whole expression again with the compiler's operations. Tested against those
+// exact: denominators in [2^-100, 2^100) (densities and pressures of any
+// unit system), numerators zero or in ±[2^-900, 2^900): velocities decay through
+// every magnitude ahead of a front. (With numerators from 2^-760 and stencils from
+// 2^-460 the 3-D shock-bubble's pre-front regions took the slow path: 163–197 ms
+// for 12 steps, now 145–183.) Violations are collected in `bad`, and the caller
+// then evaluates the whole expression again with the compiler's operations. Tested against those
 // bit for bit over both ranges.
 struct RecipRn {
     double b, y;  // b > 0
@@ -59,12 +62,14 @@ __device__ __forceinline__ double quot_rn(double a, const RecipRn& d) {
     return fma(-fma(d.b, q, -a), d.y, q);
 }
 // range tests on the high words (sign, exponent, 20 mantissa bits)
-__device__ __forceinline__ bool den_out(double b) {  // not in [2^-200, 2^200)
-    return hi_bits(b) - 0x33700000u >= 0x4c700000u - 0x33700000u;
+__device__ __forceinline__ bool den_out(double b) {  // not in [2^-100, 2^100)
+    constexpr unsigned LO = (1023u - 100u) << 20, HI = (1023u + 100u) << 20;
+    return hi_bits(b) - LO >= HI - LO;
 }
-__device__ __forceinline__ bool num_out(double a) {  // neither zero nor in ±[2^-760, 2^760)
+__device__ __forceinline__ bool num_out(double a) {  // neither zero nor in ±[2^-900, 2^900)
+    constexpr unsigned LO = (1023u - 900u) << 20, HI = (1023u + 900u) << 20;
     const unsigned h = hi_bits(a) & 0x7fffffffu;
-    return h - 0x10700000u >= 0x6f700000u - 0x10700000u && (h | (unsigned)__double2loint(a)) != 0u;
+    return h - LO >= HI - LO && (h | (unsigned)__double2loint(a)) != 0u;
 }
 __device__ __forceinline__ RecipRn den_rn(double b, bool& bad) {
     bad = bad || den_out(b);
@@ -212,12 +217,15 @@ __device__ __forceinline__ double weno5z_rn(double v0, double v1, double v2, dou
     const double s = (a0 + a1) + a2;
     // x < 2^500 (x ≥ 1e-40 by construction; a τ so small that its remainder is
     // not exact gives a ratio whose square vanishes beside 1), 16 ≤ s < 2^500
-    // (overflowed ratios and NaN fail this), 2^-460 ≤ |n| or a zero stencil
+    // (overflowed ratios and NaN fail this), |n| ≥ 2^-460, or 2^-900 for s < 2^60
+    // (the weights of values that small are the linear ones, s = 16), or a zero
+    // stencil
     const unsigned hx = max(hi_bits(x0), max(hi_bits(x1), hi_bits(x2)));
     const unsigned hn = hi_bits(n) & 0x7fffffffu;
+    const unsigned nlo = hi_bits(s) < ((1023u + 60u) << 20) ? (1023u - 900u) << 20 : 0x23300000u;
     const bool zero = (((hi_bits(Q0) | hi_bits(Q1) | hi_bits(Q2)) << 1) |
                        (unsigned)(__double2loint(Q0) | __double2loint(Q1) | __double2loint(Q2))) == 0u;
-    bad = bad || hx >= 0x5f300000u || hi_bits(s) >= 0x5f300000u || !(hn - 0x23300000u < 0x60000000u - 0x23300000u || zero);
+    bad = bad || hx >= 0x5f300000u || hi_bits(s) >= 0x5f300000u || !(hn - nlo < 0x60000000u - nlo || zero);
     return quot_rn(n, recip_sq(8.0 * s));
 }
 __device__ __forceinline__ void weno5z_pair_rn(const double* v, double& left, double& right, bool& bad) {
