@@ -34,9 +34,9 @@ CPU_STEPS = 5  # timed steps of the CPU baseline on the full grid (about 5 s eac
 AMR_STEPS = 20
 AMR_SC_STEPS = 5  # subcycled steps of the AMR sub-record (each spans about four global steps)
 CELL_BYTES_3D = 320  # algorithmic bytes per 3-D cell-update (64·F, F = 5)
-# flop per interior cell and sweep launch, counted by ncu on the 160^3 explosion
+# flop per interior cell and sweep launch, counted by ncu on the 192^3 explosion
 # (sm__sass_thread_inst_executed_op_{dadd,dmul,dfma,fadd,fmul,ffma}_pred_on, fma = 2)
-SWEEP_FLOP = {"f64": {"fp64": 2104, "fp32": 120}, "mixed": {"fp64": 464, "fp32": 750}, "fast": {"fp64": 1332, "fp32": 0}}
+SWEEP_FLOP = {"f64": {"fp64": 1823, "fp32": 0}, "mixed": {"fp64": 451, "fp32": 582}, "fast": {"fp64": 1119, "fp32": 0}}
 # FP64 pipe of a B200: 148 SMs x 64 FMA lanes x 2 flop x 1.965 GHz (nominal; no measured FP64 peak exists here)
 FP64_PEAK_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12
 
@@ -244,8 +244,7 @@ def run_ours(args, world, rank, local):
     fp64_tflops = flop["fp64"] * cells / (per_launch_ms * 1e-3) / 1e12
     fp64_roofline = {"bound": "fp64", "achieved": fp64_tflops, "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s",
                      "frac": fp64_tflops / FP64_PEAK_TFLOPS, "flop_per_cell_per_launch": flop,
-                     "flop_source": "ncu op counters, profiles/sweep_flops_uniform_160.md (plain form), "
-                                    "profiles/sweep_fast_uniform_160.md (fast and mixed forms)",
+                     "flop_source": "ncu op counters, profiles/sweep_forms_uniform_192.md",
                      "peak_source": "nominal FP64 FMA rate at 1965 MHz (148 SMs x 64 lanes x 2 flop)"}
     peaks = {}
     try:
@@ -322,9 +321,9 @@ def run_ours(args, world, rank, local):
                 "linf_vs_f64_form": [float(x) for x in np.abs(ia - ib).max(axis=0)],
                 "note": "all arithmetic FP64 with FMA contraction and Newton-refined reciprocals/square roots "
                         "(about 1 ulp) in place of correctly rounded divisions; held to 1e-12 relative L1 against "
-                        "the oracle in the parity tests; fp64_tflops_plain_equivalent counts the plain form's 2104 "
-                        "flop per cell and launch, fp64_tflops_executed the fast form's own 1332 (ncu, "
-                        "profiles/sweep_fast_uniform_160.md); both over the whole step time"}
+                        "the oracle in the parity tests; fp64_tflops_plain_equivalent counts the plain form's 1823 "
+                        "flop per cell and launch, fp64_tflops_executed the fast form's own 1119 (ncu, "
+                        "profiles/sweep_forms_uniform_192.md); both over the whole step time"}
 
     # ---- end to end through the C ABI with host buffers
     e2e = None
@@ -371,11 +370,11 @@ def run_ours(args, world, rank, local):
             "dtype": "f32-flux/f64-state" if prec == Precision.Mixed else "f64", "data": "synthetic",
             "config": dict(uniform_config(n, world, args.precision), sweep_row_loads=row_staging),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic, "traffic_source": "ncu capture on 160^3 scaled by cells (profiles/)", "kernel": "fused sweep (3 per stage)",
+                         "traffic": traffic, "traffic_source": "ncu capture on 192^3 scaled by cells (profiles/)", "kernel": "fused sweep (3 per stage)",
                          "alg_bytes_per_launch": alg_bytes_per_launch, "avg_launch_ms": per_launch_ms,
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks else "fallback",
-                         "compute_note": "the sweep is FP64-ALU bound (59 FP64 flop per algorithmic byte): FP64 pipe "
-                                         "45-50 % active at 4 CTAs per SM (ncu, profiles/sweep_flops_uniform_160.md); "
+                         "compute_note": "the sweep is FP64-ALU bound (51 FP64 flop per algorithmic byte): FP64 pipe "
+                                         "53-63 % active at 3 CTAs per SM (ncu, profiles/sweep_forms_uniform_192.md); "
                                          "the HBM fraction is small by construction",
                          "fp64": fp64_roofline},
             "kernel_ms_per_step": {k: v[0] / args.steps for k, v in kt.items()},
