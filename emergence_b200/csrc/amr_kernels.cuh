@@ -808,7 +808,7 @@ struct RefluxFace {
 // and the buckets run in the reference's (d, side) order, so every cell sums
 // its corrections in the reference's order.
 template <int NV>
-__global__ void reflux_faces(const AmrDev A, double* rhs, const double* __restrict__ face, int npen,
+__global__ void reflux_faces(const AmrDev A, double* rhs, const double* face, int npen,
                              const RefluxFace* __restrict__ tasks) {
     dependency_wait();
     dependents_may_start();
@@ -837,10 +837,17 @@ __global__ void reflux_faces(const AmrDev A, double* rhs, const double* __restri
         c[e0] = a;
         c[e1] = bb;
         double* r = rhs + (int64_t)tk.slot * A.bcell + amr_cell(A, c);
+        // every operand first: a load would otherwise wait on the stores before it
+        double df[NV], rk[NV];
+#pragma unroll
         for (int k = 0; k < NV; k++) {
-            const double df = sum[k] / cnt - fc[(int64_t)k * npen];
-            const double dr = tk.side == 1 ? -df / tk.dx : df / tk.dx;
-            r[(int64_t)k * A.ntot] = r[(int64_t)k * A.ntot] + dr;
+            df[k] = sum[k] / cnt - fc[(int64_t)k * npen];
+            rk[k] = r[(int64_t)k * A.ntot];
+        }
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const double dr = tk.side == 1 ? -df[k] / tk.dx : df[k] / tk.dx;
+            r[(int64_t)k * A.ntot] = rk[k] + dr;
         }
     }
 }
@@ -901,7 +908,7 @@ struct AmrFivePh {
 // without harm, so the sc form skips the stage-3 rate and admissibility
 // reduction; the leaves are checked by amr_cfl after the step.
 template <class PH>
-__global__ void amr_rk(const AmrDev A, double* u0, const double* __restrict__ rhs, const int* __restrict__ leaves,
+__global__ void amr_rk(const AmrDev A, double* u0, const double* rhs, const int* __restrict__ leaves,
                        const int* __restrict__ level, const double* __restrict__ dxl, int stage, StepCtl* ctl,
                        int sc) {
     dependency_wait();

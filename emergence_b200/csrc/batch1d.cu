@@ -95,7 +95,7 @@ __global__ void batch_ghosts(double* u, int64_t ntot, Inst* inst, int ninst, int
 }
 
 // CFL rate of each instance and its dt (C/solver.rs:478-523, :758-768)
-__global__ void batch_begin(const double* __restrict__ u, int64_t ntot, Inst* inst, double* dtv, int ninst, double cfl,
+__global__ void batch_begin(const double* u, int64_t ntot, Inst* inst, double* dtv, int ninst, double cfl,
                             double t_end, EosD eosd) {
     dependency_wait();
     dependents_may_start();

@@ -27,7 +27,7 @@
 namespace emg {
 
 struct FiveSweepParams {
-    const double* __restrict__ uin;
+    const double* uin;
     double* rhs;
     const double* base;
     const double* cur;
@@ -476,7 +476,7 @@ template <int P, int D, int MODE, bool AMR = false, bool FAST = false> struct Fi
                     if (s_lok[l] && in_bounds(p.ctl, g, p.ncell)) {
                         double u[NF], w[NF], d, b;
 #pragma unroll
-                        for (int k = 0; k < NF; k++) u[k] = __ldg(p.uin + k * p.ncell + g);
+                        for (int k = 0; k < NF; k++) u[k] = p.uin[k * p.ncell + g];
                         to_prim(sys, u, w, d, b);
 #pragma unroll
                         for (int k = 0; k < NF; k++) W[at<STRW>(row, k, l)] = w[k];

@@ -5,7 +5,11 @@
 // Every kernel launched this way calls dependency_wait() before it touches
 // memory that another kernel may write or still read: the call returns when all
 // earlier grids of the stream have completed and their writes are visible, so
-// the order of memory accesses is that of ordinary launches.
+// the order of memory accesses is that of ordinary launches. That holds for
+// ordinary loads only: a load through the read-only path (__ldg, or a const
+// __restrict__ pointer) promises that nobody writes the memory while the kernel
+// lives, and this kernel lives while the one before it writes. Only tables
+// uploaded before the launches may be read that way.
 // dependents_may_start() then lets the next grid be set up once every CTA of
 // this one has got that far (all of them are resident by then, so a waiting
 // grid never holds a place that a running one still needs).

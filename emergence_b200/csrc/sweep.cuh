@@ -54,7 +54,7 @@ struct StepCtl {
 };
 
 struct SweepParams {
-    const double* __restrict__ uin;  // stage input (ghost-filled along d), SoA with field stride ncell
+    const double* uin;  // stage input (ghost-filled along d), SoA with field stride ncell
     double* rhs;                     // stage residual, same indexing as uin
     const double* base;              // RK base state ("old"), last axis only
     const double* cur;               // previous value of the RK destination, last axis stages 2-3
@@ -894,7 +894,7 @@ struct Sweep {
                         const int64_t g = rowg(row) + s_loff[l];
                         double u[5], w[5];
 #pragma unroll
-                        for (int k = 0; k < 5; k++) u[k] = __ldg(p.uin + k * p.ncell + g);
+                        for (int k = 0; k < 5; k++) u[k] = p.uin[k * p.ncell + g];
                         if constexpr (FMAPS)
                             to_prim_f(ed, u, w);
                         else
