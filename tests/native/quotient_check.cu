@@ -29,6 +29,15 @@ __global__ void quotient_kernel(const double* a, const double* b, double* out, s
     o[8] = bad ? 1.0 : 0.0;
     o[9] = sqrt(b[i]);
 }
+// out per operand pair: quotient by recip_sq, a/b, flag
+__global__ void square_kernel(const double* a, const double* b, double* out, size_t n) {
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double* o = out + 3 * i;
+    o[0] = emg::quot_rn(a[i], emg::recip_sq(b[i]));
+    o[1] = a[i] / b[i];
+    o[2] = emg::sq_in(emg::lo_bits(b[i])) ? 0.0 : 1.0;
+}
 // six stencil values in; both interpolations, the plain ones, flag out
 __global__ void weno_kernel(const double* v, double* out, size_t n) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -43,15 +52,17 @@ __global__ void weno_kernel(const double* v, double* out, size_t n) {
     o[4] = bad ? 1.0 : 0.0;
 }
 
-int run(const double* in0, size_t n0, const double* in1, size_t n1, double* out_host, size_t nout, size_t n, int weno) {
+int run(const double* in0, size_t n0, const double* in1, size_t n1, double* out_host, size_t nout, size_t n, int what) {
     double *a = nullptr, *b = nullptr, *out = nullptr;
     int rc = cudaMalloc(&a, n0 * sizeof(double)) || cudaMalloc(&b, n1 * sizeof(double)) || cudaMalloc(&out, nout * sizeof(double));
     if (!rc) rc = cudaMemcpy(a, in0, n0 * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess;
     if (!rc && in1) rc = cudaMemcpy(b, in1, n1 * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess;
     if (!rc) {
         const unsigned g = (unsigned)((n + 255) / 256);
-        if (weno)
+        if (what == 1)
             weno_kernel<<<g, 256>>>(a, out, n);
+        else if (what == 2)
+            square_kernel<<<g, 256>>>(a, b, out, n);
         else
             quotient_kernel<<<g, 256>>>(a, b, out, n);
         rc = cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess;
@@ -69,3 +80,6 @@ extern "C" int quotient_check(const double* a, const double* b, double* out, siz
     return run(a, n, b, n, out, 10 * n, n, 0);
 }
 extern "C" int weno_check(const double* v, double* out, size_t n) { return run(v, 6 * n, nullptr, 1, out, 5 * n, n, 1); }
+extern "C" int square_check(const double* a, const double* b, double* out, size_t n) {
+    return run(a, n, b, n, out, 3 * n, n, 2);
+}
