@@ -9,7 +9,7 @@
 namespace emg {
 
 // dynamic shared memory of the uniform-grid kernel
-template <int P, int MODE> constexpr size_t grid_smem() {
+template <int P, int MODE> static constexpr size_t grid_smem() {
     return SweepSmem<F64Fast, P, MODE, sweep_threads<F64Fast, MODE, KIND_GRID>()>::bytes();
 }
 

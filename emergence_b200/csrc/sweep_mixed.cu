@@ -6,7 +6,7 @@
 namespace emg {
 
 // dynamic shared memory of the uniform-grid kernel
-template <int P, int MODE> constexpr size_t grid_smem() {
+template <int P, int MODE> static constexpr size_t grid_smem() {
     return SweepSmem<float, P, MODE, sweep_threads<float, MODE, KIND_GRID>()>::bytes();
 }
 
