@@ -36,7 +36,6 @@
 
 namespace emg {
 int set_error(int code, const std::string& msg);
-cudaMemPool_t state_pool(int dev);  // uniform.cu
 }
 
 using namespace emg;
@@ -2698,19 +2697,12 @@ int emg_amr_download(emg_amr* h, double* u, size_t nblocks) {
     if (!u || nblocks < h->blocks.size()) return set_error(EMG_ERR_INVALID, "buffer too small");
     const int nv = h->nv;
     const size_t n = h->blocks.size() * (size_t)h->bcells() * nv;
-    // staging from the library's pool: cudaMalloc and cudaFree of 300 MB stalled
-    // the device for up to some 100 ms per call on a shared host
-    double* tmp = nullptr;
-    cudaMemPool_t pool = state_pool(h->device);
-    if (!pool) return set_error(EMG_ERR_CUDA, "device memory pool unavailable");
-    AMR_CUDA(cudaMallocFromPoolAsync((void**)&tmp, n * sizeof(double), pool, h->stream));
+    // gathered in the residual array, which is scratch between the steps (a step's
+    // first sweep overwrites it) and at least as long: nothing is allocated
     AmrDev A = h->view();
-    NVK(pool_get_interior)<<<256, 256, 0, h->stream>>>(A, (int)h->blocks.size(), tmp);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = copy_to_host(u, tmp, n * sizeof(double), h->stream);
-    cudaFreeAsync(tmp, h->stream);
-    AMR_CUDA(e);
-    AMR_CUDA(cudaStreamSynchronize(h->stream));
+    NVK(pool_get_interior)<<<256, 256, 0, h->stream>>>(A, (int)h->blocks.size(), h->rhs);
+    AMR_CUDA(cudaGetLastError());
+    AMR_CUDA(copy_to_host(u, h->rhs, n * sizeof(double), h->stream));
     return EMG_OK;
 }
 

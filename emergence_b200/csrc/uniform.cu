@@ -1122,15 +1122,14 @@ static int check_uniform_args(const emg_mesh* mesh, const emg_bc bc[6], const em
 
 }  // extern "C"
 
-namespace emg {
-// The large state buffers of uniform-grid solvers (and the staging of block-AMR
-// downloads) come from a library-owned
+namespace {
+// The large state buffers of uniform-grid solvers come from a library-owned
 // stream-ordered memory pool per device that keeps up to 32 GB of freed
 // memory: cudaMalloc of a 256^3 state (4 GB over five buffers) costs 5-60 ms,
 // and a solver created after another one was destroyed reuses its memory.
 // emg_release_memory returns the kept memory to the device.
-static std::mutex pool_mu;
-static cudaMemPool_t pools[64] = {};
+std::mutex pool_mu;
+cudaMemPool_t pools[64] = {};
 cudaMemPool_t state_pool(int dev) {
     if (dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(pool_mu);
@@ -1150,7 +1149,7 @@ cudaMemPool_t state_pool(int dev) {
     }
     return pools[dev];
 }
-}  // namespace emg
+}  // namespace
 
 extern "C" {
 

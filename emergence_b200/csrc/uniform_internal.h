@@ -87,8 +87,6 @@ struct emg_uniform {
 
 
 namespace emg {
-// the library's stream-ordered memory pool of a device (null: unavailable)
-cudaMemPool_t state_pool(int dev);
 // ghost fill of `arr` (padded SoA) along every active axis, in axis order
 int launch_ghosts(emg_uniform* h, double* arr);
 // three SSP-RK3 stages and the time advance of one step (dt read from the control

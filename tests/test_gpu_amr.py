@@ -208,3 +208,33 @@ def test_inadmissible_leaf_state_is_reported():
     with pytest.raises(EmgError) as e:
         g.step(1e-4)
     assert e.value.code == 4
+
+
+def test_a_download_keeps_no_device_memory():
+    """A hierarchy that is downloaded and then refined has the memory it had before:
+    the download stages in the hierarchy's own arrays."""
+    import torch
+    from emergence_b200 import release_memory
+    s, cfg, lo, hi, bc, init = W.shock_bubble(dim=2, base=8, levels=3)
+    g = gpu_amr(s, cfg, lo, hi, bc, init)
+    g.step(g.dt_cfl())
+    g.download()  # kernels loaded
+    release_memory()
+    free = torch.cuda.mem_get_info()[0]
+    assert g.download().nbytes > 4 << 20
+    assert torch.cuda.mem_get_info()[0] == free
+
+
+@pytest.mark.parametrize("subcycle", [False, True])
+def test_downloads_between_steps_change_nothing(subcycle):
+    s, cfg, lo, hi, bc, init = W.shock_bubble(dim=2, base=4, levels=3, regrid_every=2)
+    a, b = (gpu_amr(s, cfg, lo, hi, bc, init, subcycle=subcycle) for _ in range(2))
+    for _ in range(5):
+        for g in (a, b):
+            if subcycle:
+                g.step_subcycled(g.dt_cfl_subcycled())
+            else:
+                g.step(g.dt_cfl())
+        first = a.download()
+        assert np.array_equal(a.download(), first)
+    assert np.array_equal(a.structure(), b.structure()) and np.array_equal(first, b.download())
