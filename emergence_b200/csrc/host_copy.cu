@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -18,6 +19,24 @@ constexpr size_t MIN_BYTES = 8u << 20;  // below this the plain copy costs less 
 std::mutex buffer_mu;  // held for the length of a staged copy: one at a time uses the buffer
 unsigned char* buffer = nullptr;
 
+// The buffer, page-locked for every device; null when there is none to be had. It
+// is host memory of the library's own that is registered with the driver, so a
+// device reset takes the page lock and not the memory: it is then locked again.
+unsigned char* locked_buffer() {
+    if (!buffer) buffer = static_cast<unsigned char*>(std::aligned_alloc(CHUNK, CHUNK * SLOTS));
+    if (!buffer) return nullptr;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, buffer) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type != cudaMemoryTypeHost && cudaHostRegister(buffer, CHUNK * SLOTS, cudaHostRegisterPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return buffer;
+}
+
 // host threads emptying the slots: at most one per two slots
 int worker_count() {
     const unsigned n = std::thread::hardware_concurrency();
@@ -27,11 +46,11 @@ int worker_count() {
 }  // namespace
 
 void release_host_buffer() {
-    std::unique_lock<std::mutex> lock(buffer_mu, std::try_to_lock);
-    if (lock.owns_lock() && buffer) {
-        cudaFreeHost(buffer);
-        buffer = nullptr;
-    }
+    std::lock_guard<std::mutex> lock(buffer_mu);  // waits for a copy that uses it
+    if (!buffer) return;
+    if (cudaHostUnregister(buffer) != cudaSuccess) cudaGetLastError();
+    std::free(buffer);
+    buffer = nullptr;
 }
 
 cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
@@ -49,11 +68,7 @@ cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t 
     std::unique_lock<std::mutex> lock(buffer_mu, std::try_to_lock);
     const int nw = worker_count();
     if (!lock.owns_lock() || nw < 2) return plain();
-    if (!buffer && cudaMallocHost((void**)&buffer, CHUNK * SLOTS) != cudaSuccess) {
-        cudaGetLastError();
-        buffer = nullptr;
-        return plain();
-    }
+    if (!locked_buffer()) return plain();
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;

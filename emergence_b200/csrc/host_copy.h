@@ -9,6 +9,6 @@
 namespace emg {
 // Queues the copy on `stream` and returns when the data is in `dst`.
 cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t stream);
-// Frees the pinned buffer if no copy is using it (emg_release_memory).
+// Frees the pinned buffer, after the copy that may be using it (emg_release_memory).
 void release_host_buffer();
 }  // namespace emg

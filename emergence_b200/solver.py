@@ -215,5 +215,6 @@ def device_count():
 
 def release_memory():
     """Give the device memory that destroyed solvers left in the library's
-    stream-ordered pools back to the device."""
+    stream-ordered pools back to the device, and the 32 MB of page-locked memory
+    that large downloads into ordinary arrays pass through back to the host."""
     check(lib().emg_release_memory())

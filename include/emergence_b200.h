@@ -155,8 +155,13 @@ int emg_uniform_create(const emg_mesh* mesh, const emg_eos* eos, const emg_bc bc
  * emg_uniform_create reuses it instead of calling the driver. */
 int emg_uniform_destroy(emg_uniform* h);
 
-/* Return the memory kept by the library's pools to the device (no Rust
- * counterpart: the reference frees through cudarc on drop). */
+/* Return the memory kept by the library to the device and the host (no Rust
+ * counterpart: the reference frees through cudarc on drop): the pools above, and
+ * 32 MB of page-locked host memory that the first download of 8 MB or more into
+ * pageable memory allocates for the process. Every download of that size passes
+ * through it, emptied by up to eight threads that live for the length of the call;
+ * one at a time uses it, others copy directly. Waits for a download that is using
+ * it. */
 int emg_release_memory(void);
 
 /* One SSP-RK3 step of size dt (G/lib.rs:402-412; C/solver.rs:659-738). */

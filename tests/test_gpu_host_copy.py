@@ -2,6 +2,9 @@
 host threads above 8 MB (emergence_b200/csrc/host_copy.cu): the same bytes as a
 direct copy into pinned memory, at sizes around the threshold and the 2 MB
 slots, and from two handles at once (needs a B200)."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -52,3 +55,33 @@ def test_released_buffer_comes_back():
     a = g.download()
     release_memory()
     assert np.array_equal(g.download(), a)
+
+
+RESET = """
+import ctypes
+import numpy as np
+from emergence_b200 import GpuAmr, GpuBatch1D, workloads as W
+
+def results():
+    sys_, n, dx, u, _ = W.riemann_batch(ninst=1024, nmax=2048)
+    b = GpuBatch1D(sys_, n, dx, u)
+    a = GpuAmr(*W.shock_bubble(dim=2, base=4, levels=2))
+    a.step(a.dt_cfl())
+    out = b.download(), a.download()
+    assert out[0].nbytes > 2 * (8 << 20)  # staged
+    b.close(), a.close()
+    return out
+
+first = results()
+assert ctypes.CDLL("libcuda.so.1").cuDevicePrimaryCtxReset_v2(0) == 0
+assert all(np.array_equal(x, y) for x, y in zip(first, results()))
+print("same")
+"""
+
+
+def test_downloads_outlive_a_device_reset():
+    """The page-locked buffer is the process's: after the context it was locked in
+    has gone, the next download locks it again."""
+    root = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..")
+    r = subprocess.run([sys.executable, "-c", RESET], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr[-2000:]
