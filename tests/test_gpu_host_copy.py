@@ -21,10 +21,14 @@ def _solver(n, seed):
     return GpuSolver(s, mesh, u, bc=bc), mesh, u
 
 
-@pytest.mark.parametrize("n", [(209690, 1, 1), (209703, 1, 1), (500, 403, 1), (64, 61, 59)])
-def test_pageable_download_equals_the_pinned_one(n):
+# bytes: 8 below the threshold, a plain copy; 32 above, four slots and a rest; sixteen
+# slots less 32 and plus 8 bytes; four slots and a bit; more than two rounds of them
+@pytest.mark.parametrize("n,staged", [((209703, 1, 1), False), ((209704, 1, 1), True), ((838848, 1, 1), True),
+                                      ((838849, 1, 1), True), ((500, 403, 1), True), ((128, 111, 119), True)])
+def test_pageable_download_equals_the_pinned_one(n, staged):
     import torch
     g, mesh, u = _solver(n, 3)
+    assert (mesh.len() * 40 >= 8 << 20) == staged
     pin = torch.empty((mesh.len(), 5), dtype=torch.float64, pin_memory=True).numpy()
     g.download(out=pin)
     out = np.full((mesh.len(), 5), np.nan)
