@@ -25,6 +25,7 @@
 #include "sweep_launch.h"
 
 #include <algorithm>
+#include <cstdlib>
 #include <array>
 #include <cmath>
 #include <cstring>
@@ -168,6 +169,7 @@ struct emg_amr {
     DevVec<RBox> dtmp_rbox;    // one-off restriction boxes (coarsened parents)
     int amrP[3] = {0, 0, 0};      // tuned pencils per CTA of the sweeps (0: default)
     bool tuned = false;
+    int chain_cap = 0;  // EMG_AMR_CHAIN: the blocks per chain (0: shorten_chains' rule)
     std::vector<PBox> pend_pbox;  // prediction boxes of refinements not yet launched
     int pend_level = -1;          // their parent level
     DevVec<double> dstage;     // host initial data of new blocks
@@ -810,7 +812,9 @@ struct emg_amr {
     // recomputes at its end. The cost is that of the uniform sweep's planner: a
     // round takes 1 + ¼(k − 1) of its time alone with k CTAs on the SM, at most
     // 3. Results do not depend on the cut (the blocks beside it exchange their
-    // values through the ghost copies again).
+    // values through the ghost copies again), so that the environment variable
+    // EMG_AMR_CHAIN may fix it: the small hierarchies that an oracle can follow are
+    // all cut to single blocks here, the large ones keep chains.
     void shorten_chains(int d, std::vector<int>& off) const {
         int o[2], no = 0;
         for (int e = 0; e < 3; e++)
@@ -820,9 +824,9 @@ struct emg_amr {
         const int P = amr_sweep_P(d, lane, other), lw = std::min(P, bd[lane]), RM = SWEEP_THREADS / P;
         const int64_t groups = (bd[other] + P / lw - 1) / (P / lw), sms = 148, slots = 3 * sms;
         auto shared = [](int64_t k) { return 1.0 + 0.25 * (double)(k - 1); };
-        int best = AMR_CHAIN_MAX;
+        int best = chain_cap ? chain_cap : AMR_CHAIN_MAX;
         double best_cost = 1e300;
-        for (int cap = AMR_CHAIN_MAX; cap >= 1; cap /= 2) {
+        for (int cap = AMR_CHAIN_MAX; cap >= 1 && !chain_cap; cap /= 2) {
             // rounds of all CTAs, and of the longest: the waves' total against the critical path
             int64_t ctas = 0, work = 0, longest = 0;
             for (size_t c = 0; c + 1 < off.size(); c++)
@@ -2400,6 +2404,7 @@ struct emg_amr {
         std::memset(ctl_host, 0, sizeof(StepCtl));
         ctl_host->t_end = INFINITY;
         AMR_CUDA(cudaMemcpy(ctl, ctl_host, sizeof(StepCtl), cudaMemcpyHostToDevice));
+        if (const char* c = std::getenv("EMG_AMR_CHAIN")) chain_cap = std::max(0, std::min(AMR_CHAIN_MAX, std::atoi(c)));
         int rc = ddxl.put(dxl, stream);
         if (rc) return rc;
         if (sweep_prepare_device() != cudaSuccess) return set_error(EMG_ERR_CUDA, "sweep setup failed");
