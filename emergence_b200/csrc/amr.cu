@@ -141,6 +141,7 @@ struct emg_amr {
     uint64_t faces = 0, weno_faces = 0;
     // ---- device
     int device = 0;
+    int64_t sms = 148;          // of the device
     cudaStream_t stream = nullptr;
     int64_t bcell = 0, cap = 0;  // pool capacity in blocks
     double *u = nullptr, *u0 = nullptr, *rhs = nullptr, *face = nullptr;
@@ -811,10 +812,12 @@ struct emg_amr {
     // leave SMs idle; on a large one shorter chains only add the 5 rows each
     // recomputes at its end. The cost is that of the uniform sweep's planner: a
     // round takes 1 + ¼(k − 1) of its time alone with k CTAs on the SM, at most
-    // 3. Results do not depend on the cut (the blocks beside it exchange their
-    // values through the ghost copies again), so that the environment variable
-    // EMG_AMR_CHAIN may fix it: the small hierarchies that an oracle can follow are
-    // all cut to single blocks here, the large ones keep chains.
+    // 3. (Of the five-equation sweeps 2 fit, but counting 2 chose longer chains and was
+    // slower: 1098 leaves in 2-D 1.85 → 2.01 ms per step, 132 in 3-D 3.55 → 3.89.)
+    // Results do not depend on the cut (the blocks beside it exchange their values
+    // through the ghost copies again), so that the environment variable EMG_AMR_CHAIN
+    // may fix it: the small hierarchies that an oracle can follow are all cut to
+    // single blocks here, the large ones keep chains.
     void shorten_chains(int d, std::vector<int>& off) const {
         int o[2], no = 0;
         for (int e = 0; e < 3; e++)
@@ -822,7 +825,7 @@ struct emg_amr {
         int lane = o[1], other = o[0];
         if (!act[lane] && act[other]) std::swap(lane, other);
         const int P = amr_sweep_P(d, lane, other), lw = std::min(P, bd[lane]), RM = SWEEP_THREADS / P;
-        const int64_t groups = (bd[other] + P / lw - 1) / (P / lw), sms = 148, slots = 3 * sms;
+        const int64_t groups = (bd[other] + P / lw - 1) / (P / lw), resident = 3, slots = resident * sms;
         auto shared = [](int64_t k) { return 1.0 + 0.25 * (double)(k - 1); };
         int best = chain_cap ? chain_cap : AMR_CHAIN_MAX;
         double best_cost = 1e300;
@@ -837,8 +840,8 @@ struct emg_amr {
                     longest = std::max(longest, r);
                 }
             if (!ctas) return;
-            const double load = (double)work / (double)slots * shared(3);
-            const double path = (double)longest * shared(std::min<int64_t>(3, (ctas + sms - 1) / sms));
+            const double load = (double)work / (double)slots * shared(resident);
+            const double path = (double)longest * shared(std::min(resident, (ctas + sms - 1) / sms));
             const double cost = std::max(load, path);
             if (cost < best_cost * 0.95) {
                 best_cost = cost;
@@ -1195,7 +1198,9 @@ struct emg_amr {
         }
         cudaEventDestroy(a);
         cudaEventDestroy(b);
-        return rc;
+        if (rc) return rc;
+        layout_valid = false;  // the chains are cut for the pencils per CTA
+        return ensure_layout();
     }
 
     int compute_rhs(int stage) {
@@ -2396,6 +2401,7 @@ struct emg_amr {
         cudaDeviceProp pr;
         AMR_CUDA(cudaGetDeviceProperties(&pr, device));
         if (pr.major != 10) return set_error(EMG_ERR_NO_DEVICE, "device is not sm_100 (B200)");
+        sms = pr.multiProcessorCount;
         AMR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         AMR_CUDA(cudaMalloc(&err, sizeof(unsigned int)));
         AMR_CUDA(cudaMemset(err, 0, sizeof(unsigned int)));
