@@ -141,15 +141,16 @@ int sweep_tma_ctas_per_sm_f64() {
     return n;
 }
 
-// resident CTAs per SM of the uniform-grid sweep (the three axes share registers and shared memory)
+// resident CTAs per SM of the uniform-grid sweep (the three axes share registers and
+// shared memory); 0: not known
 template <int P, int MODE> static int occupancy() {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_f64_kernel<P, 0, MODE>, SWEEP_THREADS,
                                                       SweepSmem<double, P, MODE>::bytes()) != cudaSuccess) {
         cudaGetLastError();
-        return 1;
+        return 0;
     }
-    return n > 0 ? n : 1;
+    return n;
 }
 template <int MODE> static int occupancy_p(int P) {
     return P == 8 ? occupancy<8, MODE>() : (P == 16 ? occupancy<16, MODE>() : occupancy<32, MODE>());

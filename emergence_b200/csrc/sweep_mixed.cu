@@ -148,15 +148,16 @@ int sweep_tma_ctas_per_sm_mixed() {
     return n;
 }
 
-// resident CTAs per SM of the uniform-grid sweep (the three axes share registers and shared memory)
+// resident CTAs per SM of the uniform-grid sweep (the three axes share registers and
+// shared memory); 0: not known
 template <int P, int MODE> static int occupancy() {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_mixed_kernel<P, 0, MODE>, sweep_threads<float, MODE, KIND_GRID>(),
                                                       grid_smem<P, MODE>()) != cudaSuccess) {
         cudaGetLastError();
-        return 1;
+        return 0;
     }
-    return n > 0 ? n : 1;
+    return n;
 }
 template <int MODE> static int occupancy_p(int P) {
     return P == 8 ? occupancy<8, MODE>() : (P == 16 ? occupancy<16, MODE>() : occupancy<32, MODE>());

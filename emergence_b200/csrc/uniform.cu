@@ -539,14 +539,14 @@ static int sweep_cta_threads(const emg_uniform* h) {
 }
 
 // Cost of sweeping along d with P pencils per CTA and segments of `seg` cells,
-// in rounds of a CTA that has its SM to itself. A CTA computes RM = threads/P
+// in rounds of a CTA of T threads that has its SM to itself. A CTA computes RM = T/P
 // midpoints of every pencil per round and seg + 5 of them in all; a round takes
 // longer the more warps share the SM's FP64 pipe (a 256-thread CTA alone about
 // 9 µs in the plain form, three of them 13.6 µs: 256³, 33 rounds); beyond 24
 // warps CTAs wait for a slot.
-static double sweep_cost(const emg_uniform* h, int d, int P, int64_t seg, int sms, int per_sm) {
+static double sweep_cost(const emg_uniform* h, int d, int P, int64_t seg, int sms, int T, int per_sm) {
     const int64_t nd = h->mesh.n[d], pencils = h->mesh.n[h->lane_axis[d]] * h->mesh.n[h->other_axis[d]];
-    const int T = sweep_cta_threads(h), RM = T / P;
+    const int RM = T / P;
     const int64_t ctas = (pencils + P - 1) / P * ((nd + seg - 1) / seg), slots = (int64_t)sms * per_sm;
     const double rounds = (double)((seg + 5 + RM - 1) / RM);
     auto shared = [&](int64_t k) { return 1.0 + 0.25 * std::max<double>(0.0, (double)k * T / SWEEP_THREADS - 1.0); };
@@ -556,8 +556,9 @@ static double sweep_cost(const emg_uniform* h, int d, int P, int64_t seg, int sm
 
 // Segment length of the sweep along d with P pencils per CTA, and its cost:
 // short segments fill the SMs on small grids, long ones save halo rows; a
-// shorter segment is taken only when it is 5 % cheaper.
-int64_t plan_seg(const emg_uniform* h, int d, int P, double* cost_out) {
+// shorter segment is taken only when it is 5 % cheaper. `T` and `resident`: threads
+// of a CTA and CTAs per SM, where they are not those of the form's plain-load kernel.
+int64_t plan_seg(const emg_uniform* h, int d, int P, double* cost_out, int T = 0, int resident = 0) {
     const int64_t nd = h->mesh.n[d];
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
@@ -567,24 +568,27 @@ int64_t plan_seg(const emg_uniform* h, int d, int P, double* cost_out) {
     // at most 3 resident CTAs of 256 threads per SM count as slots: a fourth shares
     // the SM's FP64 pipe instead of adding throughput, so cutting pencils into
     // shorter segments to fill it only adds halo rows
-    // (the kernels and the devices are the same for every handle: asked once)
-    static std::atomic<int> known[3][3][3];
-    std::atomic<int>& slot = known[h->opts.precision][h->opts.mode][P == 8 ? 0 : (P == 16 ? 1 : 2)];
-    int resident = slot.load(std::memory_order_relaxed);
+    // (what fits is the kernel's and the device's: asked once, unless the answer failed)
+    if (!T) T = sweep_cta_threads(h);
     if (!resident) {
-        resident = h->opts.precision == EMG_PRECISION_MIXED      ? sweep_ctas_per_sm_mixed(P, h->opts.mode)
-                   : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_ctas_per_sm_fast(P, h->opts.mode)
-                                                                 : sweep_ctas_per_sm_f64(P, h->opts.mode);
-        slot.store(resident, std::memory_order_relaxed);
+        static std::atomic<int> known[64][3][3][3];
+        std::atomic<int>* slot = dev >= 0 && dev < 64 ? &known[dev][h->opts.precision][h->opts.mode][P == 8 ? 0 : (P == 16 ? 1 : 2)] : nullptr;
+        if (slot) resident = slot->load(std::memory_order_relaxed);
+        if (!resident) {
+            resident = h->opts.precision == EMG_PRECISION_MIXED      ? sweep_ctas_per_sm_mixed(P, h->opts.mode)
+                       : h->opts.precision == EMG_PRECISION_F64_FAST ? sweep_ctas_per_sm_fast(P, h->opts.mode)
+                                                                     : sweep_ctas_per_sm_f64(P, h->opts.mode);
+            if (slot && resident) slot->store(resident, std::memory_order_relaxed);
+        }
     }
-    const int per_sm = std::min(3 * SWEEP_THREADS / sweep_cta_threads(h), resident);
+    const int per_sm = std::max(1, std::min(3 * SWEEP_THREADS / T, resident));
     int64_t best = nd;
     double best_cost = 1e300;
     for (int64_t k = 1; k <= nd && k <= 65535; k++) {
         const int64_t seg = (nd + k - 1) / k;
         if (k > 1 && seg < 16) break;
         if ((nd + seg - 1) / seg != k) continue;  // same seg as a smaller k
-        const double cost = sweep_cost(h, d, P, seg, sms, per_sm);
+        const double cost = sweep_cost(h, d, P, seg, sms, T, per_sm);
         if (cost < best_cost * 0.95) {
             best_cost = cost;
             best = seg;
@@ -770,7 +774,7 @@ void setup_tma(emg_uniform* h) {
     for (int d = 0; d < 3; d++)
         if (h->active[d] && h->sweepP[d] < 32 && h->mesh.n[h->lane_axis[d]] > 16) {
             h->sweepP[d] = 32;
-            h->sweepSeg[d] = (int)plan_seg(h, d, 32, nullptr);
+            h->sweepSeg[d] = (int)plan_seg(h, d, 32, nullptr, SWEEP_THREADS, staged);
             h->sweepGrid[d] = sweep_grid(h, d, 32, h->sweepSeg[d]);
         }
 }
