@@ -10,6 +10,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
+#include <string.h>
 
 namespace emg {
 
@@ -61,6 +62,17 @@ __device__ __forceinline__ float rsqrt_(float x) { return sqrtf(x); }
 __device__ __forceinline__ double rabs(double x) { return fabs(x); }
 __device__ __forceinline__ float rabs(float x) { return fabsf(x); }
 
+// high word: sign, exponent, 20 bits of the significand
+__device__ __forceinline__ unsigned hi_bits(double x) {
+#ifdef __CUDACC__
+    return (unsigned)__double2hiint(x);
+#else  // host build of the tests
+    unsigned long long b;
+    memcpy(&b, &x, sizeof b);
+    return (unsigned)(b >> 32);
+#endif
+}
+
 // Euler system, w = (ρ,u,v,w,p), u = (ρ,ρu,ρv,ρw,E): system.rs:196-217.
 template <typename R> __device__ __forceinline__ void to_prim(const Eos<R>& e, const R* u, R* w) {
     R rho = u[0];
@@ -88,6 +100,25 @@ template <typename R> __device__ __forceinline__ R sound_speed(const Eos<R>& e, 
 // system.rs:404-407 with eos.rs:75-79
 template <typename R> __device__ __forceinline__ bool admissible(const Eos<R>& e, R rho, R p) {
     return isfinite(rho) && isfinite(p) && rho > R(0) && R(1) / rho > e.b && p + e.p_inf > R(0);
+}
+// Division-free sufficient condition for the admissibility test of a
+// conserved state a of an ideal gas (b = q = p∞ = 0): ρ > 0 and
+// 2ρE − |ρu|² > 0 with a relative margin of 1e-11, values bounded so that
+// nothing over- or underflows. Whenever it holds, the reference's test
+// (to_prim: ein = E/ρ − ½|u|², p = (γ−1)·ein/(1/ρ); then ρ > 0, p > 0,
+// both finite, 1/ρ > 0) holds as well: the computed ein is within a few
+// ulps of (2ρE − |ρu|²)/(2ρ²), far inside the margin, as are the roundings
+// of this test. Where it does not hold, the reference's test runs as is, so
+// the decision is always the reference's. The bounds (2^±332) and the sign
+// are tested on the high words, off the FP64 pipe.
+__device__ __forceinline__ bool surely_admissible(const double* a) {
+    const unsigned hr = hi_bits(a[0]), hE = hi_bits(a[4]);
+    const unsigned h1 = hi_bits(a[1]) & 0x7fffffffu, h2 = hi_bits(a[2]) & 0x7fffffffu, h3 = hi_bits(a[3]) & 0x7fffffffu;
+    const unsigned h12 = h1 > h2 ? h1 : h2, hm = h12 > h3 ? h12 : h3;
+    constexpr unsigned LO = (1023u - 332u) << 20, HI = (1023u + 332u) << 20;
+    const double m2 = fma(a[3], a[3], fma(a[2], a[2], a[1] * a[1]));
+    const double d = fma(2.0 - 2e-11, a[0] * a[4], -(1.0 + 1e-11) * m2);
+    return hr - LO < HI - LO && hE - LO < HI - LO && hm < HI && (int)hi_bits(d) > 0;
 }
 // physical flux from primitive w and its conserved q along normal index un (system.rs:268-278)
 template <typename R> __device__ __forceinline__ void flux_wq(const R* w, const R* q, int un, R* f) {

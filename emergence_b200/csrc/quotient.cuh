@@ -31,7 +31,6 @@ namespace emg {
 struct RecipRn {
     double b, y;  // b > 0
 };
-__device__ __forceinline__ unsigned hi_bits(double x) { return (unsigned)__double2hiint(x); }
 // y = RN(1/b): the PTX estimate r (2^-20), the series step r·(1 + h + h²)
 // (2^-60 before its rounding, so a faithful reciprocal), and Markstein's
 // correction, which rounds every reciprocal correctly but that of an all-ones

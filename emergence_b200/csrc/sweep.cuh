@@ -587,25 +587,6 @@ struct Sweep {
         }
     }
 
-    // Division-free sufficient condition for the admissibility test of a
-    // conserved state a of an ideal gas (b = q = p∞ = 0): ρ > 0 and
-    // 2ρE − |ρu|² > 0 with a relative margin of 1e-11, values bounded so that
-    // nothing over- or underflows. Whenever it holds, the reference's test
-    // (to_prim: ein = E/ρ − ½|u|², p = (γ−1)·ein/(1/ρ); then ρ > 0, p > 0,
-    // both finite, 1/ρ > 0) holds as well: the computed ein is within a few
-    // ulps of (2ρE − |ρu|²)/(2ρ²), far inside the margin, as are the roundings
-    // of this test. Where it does not hold, the reference's test runs as is, so
-    // the decision is always the reference's. The bounds (2^±332) and the sign
-    // are tested on the high words, off the FP64 pipe.
-    __device__ static __forceinline__ bool surely_admissible(const double* a) {
-        const unsigned hr = hi_bits(a[0]), hE = hi_bits(a[4]);
-        const unsigned hm = max(hi_bits(a[1]) & 0x7fffffffu, max(hi_bits(a[2]) & 0x7fffffffu, hi_bits(a[3]) & 0x7fffffffu));
-        constexpr unsigned LO = (1023u - 332u) << 20, HI = (1023u + 332u) << 20;
-        const double m2 = fma(a[3], a[3], fma(a[2], a[2], a[1] * a[1]));
-        const double d = fma(2.0 - 2e-11, a[0] * a[4], -(1.0 + 1e-11) * m2);
-        return hr - LO < HI - LO && hE - LO < HI - LO && hm < HI && __double2hiint(d) > 0;
-    }
-
     // one-sided admissibility of the limiter (C/scheme.rs:408-416), in f64;
     // `ideal`: the equation of state is an ideal gas with 1 < γ < 100, which
     // admits the division-free test above

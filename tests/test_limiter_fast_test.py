@@ -1,20 +1,32 @@
 """The division-free admissibility test that the sweep's positivity limiter
-tries first (Sweep::surely_admissible, ideal gas) never accepts a state that
-the reference's test (to_prim then admissible, C/system.rs:197-203,404-407)
-rejects, so the limiter decides exactly as the reference does. Restated here
-with numpy in the same IEEE double operations (host, no GPU), over states
+tries first (surely_admissible of emergence_b200/csrc/physics.cuh, ideal gas) never
+accepts a state that the reference's test (to_prim then admissible,
+C/system.rs:197-203,404-407) rejects, so the limiter decides exactly as the
+reference does. The function itself, compiled for the host (no GPU), over states
 spread across the admissibility boundary."""
+import ctypes as C
+import os
+import subprocess
+
 import numpy as np
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SRC = os.path.join(HERE, "native", "admissible_host.cpp")
+OUT = os.path.join(HERE, "native", "_build", "libadmissible_host.so")
+DEPS = [SRC, os.path.join(HERE, "..", "emergence_b200", "csrc", "physics.cuh")]
 
 
 def surely_admissible(a):
-    r, E = a[:, 0], a[:, 4]
-    ok = (r > 1e-100) & (r < 1e100) & (E > 1e-100) & (E < 1e100)
-    for k in (1, 2, 3):
-        ok &= np.abs(a[:, k]) < 1e100
-    m2 = a[:, 1] * a[:, 1] + a[:, 2] * a[:, 2] + a[:, 3] * a[:, 3]
-    twore = 2.0 * r * E
-    return ok & (twore - m2 > 1e-11 * (twore + m2))
+    os.makedirs(os.path.dirname(OUT), exist_ok=True)
+    if not os.path.exists(OUT) or any(os.path.getmtime(d) > os.path.getmtime(OUT) for d in DEPS):
+        cuda_inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+        subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-Wno-unknown-pragmas",
+                        "-I", cuda_inc, SRC, "-o", OUT], check=True)
+    a = np.ascontiguousarray(a, dtype=np.float64)
+    out = np.zeros(len(a), dtype=np.uint8)
+    lib = C.CDLL(OUT)
+    lib.admissible_check(C.c_void_p(a.ctypes.data), C.c_size_t(len(a)), C.c_void_p(out.ctypes.data))
+    return out.astype(bool)
 
 
 def reference_admissible(a, gamma):
@@ -66,3 +78,14 @@ def test_fast_test_rejects_extremes_and_non_finite_values():
                   [1.0, 0, 0, 0, np.inf],
                   [1e-200, 0, 0, 0, 1e-200]])   # outside the bounded range: left to the full test
     assert list(surely_admissible(a)) == [True, False, False, False, False, False, False]
+
+
+def test_fast_test_bounds():
+    """2^±332 on ρ, E and |ρu|: beyond them the test leaves the state to the full one."""
+    lo, hi = 2.0 ** -332, 2.0 ** 332
+    below = np.nextafter
+    ok = np.array([[lo, 0, 0, 0, 1.0], [1.0, 0, 0, 0, lo], [below(hi, 0), 0, 0, 0, 1.0], [below(hi, 0), 0, 0, 0, below(hi, 0)],
+                   [below(hi, 0), 0, -below(hi, 0), 0, below(hi, 0)]])
+    out = np.array([[below(lo, 0), 0, 0, 0, 1.0], [1.0, 0, 0, 0, below(lo, 0)], [hi, 0, 0, 0, 1.0], [1.0, 0, 0, 0, hi],
+                    [1.0, hi, 0, 0, 1.0], [1.0, 0, -hi, 0, 1.0], [1.0, 0, 0, np.nan, 1.0], [1.0, 0, 0, -np.inf, 1.0]])
+    assert surely_admissible(ok).all() and not surely_admissible(out).any()
