@@ -262,46 +262,25 @@ __device__ __forceinline__ double hllc_fs(const Eos<double>& e, const double* wl
     return ss;
 }
 
-// WENO-Z combination (scheme.rs:76-86); eps 1e-40 in f64 (scheme.rs:55), 1e-30 in f32.
-template <typename R> struct WenoEps;
-template <> struct WenoEps<double> { static constexpr double v = 1e-40; };
-template <> struct WenoEps<float> { static constexpr float v = 1e-30f; };
+// WENO-Z combination (scheme.rs:76-86), eps of scheme.rs:55
+constexpr double WENO_EPS = 1e-40;
 
 template <typename R> __device__ __forceinline__ R sq(R x) { return x * x; }
 
 // WENO5-Z interpolation of point values to the midpoint x_{2+1/2} (scheme.rs:67-74).
-// The FP32 instance is the host restatement's (the mixed sweep uses weno5z_pair_m).
-template <typename R> __device__ __forceinline__ R weno5z_interp(R v0, R v1, R v2, R v3, R v4) {
-    const R eps = WenoEps<R>::v;
+__device__ __forceinline__ double weno5z_interp(double v0, double v1, double v2, double v3, double v4) {
     // x/8 == x*0.125 exactly (power-of-two scaling)
-    R q0 = (R(3) * v0 - R(10) * v1 + R(15) * v2) * R(0.125);
-    R q1 = (-v1 + R(6) * v2 + R(3) * v3) * R(0.125);
-    R q2 = (R(3) * v2 + R(6) * v3 - v4) * R(0.125);
-    R b0 = R(13.0 / 12.0) * sq(v0 - R(2) * v1 + v2) + R(0.25) * sq(v0 - R(4) * v1 + R(3) * v2);
-    R b1 = R(13.0 / 12.0) * sq(v1 - R(2) * v2 + v3) + R(0.25) * sq(v1 - v3);
-    R b2 = R(13.0 / 12.0) * sq(v2 - R(2) * v3 + v4) + R(0.25) * sq(R(3) * v2 - R(4) * v3 + v4);
-    R tau = rabs(b0 - b2);
-    if constexpr (sizeof(R) == 4) {
-        // FP32: the reference weights a_k = d_k (1 + (τ/(β_k+ε))²) overflow when a
-        // stencil is flat (β_k = 0: (1e-6/1e-30)² = 1e48 > FLT_MAX) and the
-        // interpolant turns NaN. Scale every a_k by (m/t)², m = min_k(β_k+ε),
-        // t = max(τ, m): identical weights in exact arithmetic, all terms ≤ 2 d_k.
-        const R b0e = b0 + eps, b1e = b1 + eps, b2e = b2 + eps;
-        const R m = rmin(b0e, rmin(b1e, b2e));
-        const R t = rmax(tau, m);
-        const R g = m / t, h = tau / t;
-        const R r0 = (m / b0e) * h, r1 = (m / b1e) * h, r2 = (m / b2e) * h;
-        const R g2 = g * g;
-        const R a0 = R(1.0 / 16.0) * (g2 + r0 * r0);
-        const R a1 = R(10.0 / 16.0) * (g2 + r1 * r1);
-        const R a2 = R(5.0 / 16.0) * (g2 + r2 * r2);
-        return (a0 * q0 + a1 * q1 + a2 * q2) / (a0 + a1 + a2);
-    } else {
-        R a0 = R(1.0 / 16.0) * (R(1) + sq(tau / (b0 + eps)));
-        R a1 = R(10.0 / 16.0) * (R(1) + sq(tau / (b1 + eps)));
-        R a2 = R(5.0 / 16.0) * (R(1) + sq(tau / (b2 + eps)));
-        return (a0 * q0 + a1 * q1 + a2 * q2) / (a0 + a1 + a2);
-    }
+    const double q0 = (3.0 * v0 - 10.0 * v1 + 15.0 * v2) * 0.125;
+    const double q1 = (-v1 + 6.0 * v2 + 3.0 * v3) * 0.125;
+    const double q2 = (3.0 * v2 + 6.0 * v3 - v4) * 0.125;
+    const double b0 = (13.0 / 12.0) * sq(v0 - 2.0 * v1 + v2) + 0.25 * sq(v0 - 4.0 * v1 + 3.0 * v2);
+    const double b1 = (13.0 / 12.0) * sq(v1 - 2.0 * v2 + v3) + 0.25 * sq(v1 - v3);
+    const double b2 = (13.0 / 12.0) * sq(v2 - 2.0 * v3 + v4) + 0.25 * sq(3.0 * v2 - 4.0 * v3 + v4);
+    const double tau = rabs(b0 - b2);
+    const double a0 = (1.0 / 16.0) * (1.0 + sq(tau / (b0 + WENO_EPS)));
+    const double a1 = (10.0 / 16.0) * (1.0 + sq(tau / (b1 + WENO_EPS)));
+    const double a2 = (5.0 / 16.0) * (1.0 + sq(tau / (b2 + WENO_EPS)));
+    return (a0 * q0 + a1 * q1 + a2 * q2) / (a0 + a1 + a2);
 }
 
 // ------------------------------------------------------------------ fast FP64 form

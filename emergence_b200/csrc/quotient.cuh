@@ -207,7 +207,6 @@ __device__ __forceinline__ void hllc_rn(const Eos<double>& e, const RecipRn& rg,
 // one side; t2 = RN(3·v2), t3 = RN(3·v3)
 __device__ __forceinline__ double weno5z_rn(double v0, double v1, double v2, double v3, double v4, double t2, double t3,
                                             bool& bad) {
-    const double eps = WenoEps<double>::v;
     // 8·q_k: 6x = 2·RN(3x) exactly
     const double Q0 = (3.0 * v0 - 10.0 * v1) + 15.0 * v2;
     const double Q1 = fma(2.0, t2, -v1) + t3;
@@ -220,7 +219,7 @@ __device__ __forceinline__ double weno5z_rn(double v0, double v1, double v2, dou
     const double b1 = fma(0.25, sq(B1), (13.0 / 12.0) * sq(D1));
     const double b2 = fma(0.25, sq(B2), (13.0 / 12.0) * sq(D2));
     const double tau = fabs(b0 - b2);
-    const double x0 = b0 + eps, x1 = b1 + eps, x2 = b2 + eps;
+    const double x0 = b0 + WENO_EPS, x1 = b1 + WENO_EPS, x2 = b2 + WENO_EPS;
     const double a0 = 1.0 + sq(quot_rn(tau, recip_sq(x0)));
     const double a1 = 10.0 * (1.0 + sq(quot_rn(tau, recip_sq(x1))));
     const double a2 = 5.0 * (1.0 + sq(quot_rn(tau, recip_sq(x2))));
