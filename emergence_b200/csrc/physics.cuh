@@ -5,8 +5,7 @@
 // Formulas and their operation order follow the reference CPU solver
 // (fluid/crates/compressible/src/{eos,system,scheme}.rs) so that the plain FP64
 // instantiation, compiled without FMA contraction, rounds exactly as the CPU
-// does. The same templates instantiated with R = float give the FP32 flux
-// arithmetic of the mixed-precision form.
+// does. The mixed form takes its FP32 sound speeds from the same templates.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -471,7 +470,9 @@ __device__ __forceinline__ void weno5z_pair_f(const double* v, double& left, dou
 // weights 1 + (τ/x_k)² would overflow on a flat stencil (x_k = 4e-30) and their
 // multiples by (x0x1x2)² underflow, so each is scaled by (m/t)², m = min x_k,
 // t = max(τ, m): all terms are at most 2. The correction to the centre is added
-// in FP64.
+// in FP64. x_k = 4β_k stays below 2^126 for differences up to about 2e18; beyond, the
+// result is not finite and the midpoint falls back to the cell averages (as it did
+// from twice that with β_k in place of 4β_k).
 __device__ __forceinline__ float weno5z_side_m(float x0, float x1, float x2, float e0, float e1, float e2) {
     const float tau = fabsf(x0 - x2);
     const float m = fminf(x0, fminf(x1, x2));

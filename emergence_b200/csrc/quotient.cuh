@@ -26,8 +26,8 @@ namespace emg {
 // every magnitude ahead of a front. (With numerators from 2^-760 and stencils from
 // 2^-460 the 3-D shock-bubble's pre-front regions took the slow path: 163–197 ms
 // for 12 steps, now 145–183.) Violations are collected in `bad`, and the caller
-// then evaluates the whole expression again with the compiler's operations. Tested against those
-// bit for bit over both ranges.
+// then evaluates the whole expression again with the compiler's operations. Tested
+// against those bit for bit over both ranges.
 struct RecipRn {
     double b, y;  // b > 0
 };
@@ -201,8 +201,8 @@ __device__ __forceinline__ void hllc_rn(const Eos<double>& e, const RecipRn& rg,
 // sweep has ten interpolations and some twenty more quotients and roots): 256³
 // explosion step, plain form, 23.6 → 18.5 ms; 4096 batched lines, 20 steps of
 // the longest, 67.7 → 49.4 ms; five-equation 96³ step 6.4 → 4.3 ms; 48² single
-// step 0.31 → 0.20 ms. FP64 pipe instructions per cell and sweep 1724 → 1480;
-// what bounds the sweep now is that pipe (about 60 % busy at 24 warps per SM)
+// step 0.31 → 0.20 ms. FP64 pipe instructions per cell and sweep 1724 → 1338;
+// what bounds the sweep now is that pipe (53–63 % active at 24 warps per SM)
 // and the latency of the chains that feed it.
 // one side; t2 = RN(3·v2), t3 = RN(3·v3)
 __device__ __forceinline__ double weno5z_rn(double v0, double v1, double v2, double v3, double v4, double t2, double t3,

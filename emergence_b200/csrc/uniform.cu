@@ -734,8 +734,8 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 // TMA row staging is an explicit opt-in (EMG_TMA=1): it is used wherever its
-// alignment conditions hold, although its staging tile leaves room for fewer
-// resident CTAs per SM (3) than the plain-load sweeps (4)
+// alignment conditions hold, although it measures no faster than the plain loads
+// (190×170×150: 6.31 against 6.16 ms per step, mixed 4.17 against 3.52)
 void setup_tma(emg_uniform* h) {
     h->tma = 0;
     const char* on = std::getenv("EMG_TMA");
