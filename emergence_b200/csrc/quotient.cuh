@@ -46,27 +46,22 @@ __device__ __forceinline__ RecipRn recip_rn(double b) {
     return RecipRn{b, __hiloint2double(__double2hiint(r), __double2loint(r) + (ones ? 1 : 0))};
 }
 // One operation less, for sums of squares: two Newton steps, so y is within (½ + ε)
-// ulp of 1/b, not always RN(1/b). quot_rn of it is RN(a/b) for every b < 2 − 4ε
-// (scaled to [1, 2)): for an a/b next to a midpoint q is half an ulp away, so q + r·y
-// is off by at most b·(1 + 2ε)·2^-55 ulp(q), while a/b keeps 2^-53/b ulp(q) from the
-// midpoint, and b²(1 + 2ε) < 4; and for a q = RN(a·y) more than an ulp off there,
-// a·(½ + ε) ≥ 1 − 2^-52, so b > a > 2 − 4ε. The estimate is good to 2^-19.9, which
-// makes ε = 2^-26; it is exactly ½ for b = 2 − δ, δ ≤ 2^-20, so ε = 2^48·δ⁴ + 2^-53
-// there, and only a δ of a few 2^-52 is left. It does go wrong (a = 2, b = 2 − 2^-52),
-// and sq_in, which the caller tests, keeps well away from it.
+// ulp of 1/b, not always RN(1/b). quot_rn of it is RN(a/b) all the same, by its error
+// for b < 2 − 4ε (scaled to [1, 2)): for an a/b next to a midpoint q is half an ulp
+// away, so q + r·y is off by at most b·(1 + 2ε)·2^-55 ulp(q), while a/b keeps 2^-53/b
+// ulp(q) from the midpoint, and b²(1 + 2ε) < 4; and for a q = RN(a·y) more than an ulp
+// off there, a·(½ + ε) ≥ 1 − 2^-52, so b > a > 2 − 4ε. The estimate is good to 2^-19.9,
+// which makes ε = 2^-26. For b = 2 − δ, δ ≤ 2^-20, the estimate is exactly ½ and
+// ε = 2^48·δ⁴ + δ²/2 + 2^-52, so only δ = k·2^-52, k ≤ 4, is left, and there y = RN(1/b):
+// the first step gives ½ + k·2^-54, for an odd k halfway between two values and
+// rounded up, so that the second step sees 1/b's next term (rounded to nearest, k = 1
+// stays at ½ in both steps and 2/b comes out as 1).
 __device__ __forceinline__ RecipRn recip_sq(double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    r = fma(r, fma(-b, r, 1.0), r);
+    r = __fma_ru(r, fma(-b, r, 1.0), r);
     return RecipRn{b, fma(r, fma(-b, r, 1.0), r)};
 }
-// The low words of the denominators tell: the 256 values below 2 have one of
-// 0xffffff00 or above (as has one of 2^24 others, which then take the slow path for
-// nothing), so the largest low word of several denominators tests them all. Three
-// integer operations for the four of an interpolation; testing the high words as well
-// took 256³ from 122.7 to 125.0 ms.
-__device__ __forceinline__ unsigned lo_bits(double x) { return (unsigned)__double2loint(x); }
-__device__ __forceinline__ bool sq_in(unsigned lo) { return lo < 0xffffff00u; }
 // a/b without checks; the remainder's sign keeps the sign of a zero numerator
 __device__ __forceinline__ double quot_rn(double a, const RecipRn& d) {
     const double q = a * d.y;
@@ -229,14 +224,13 @@ __device__ __forceinline__ double weno5z_rn(double v0, double v1, double v2, dou
     // not exact gives a ratio whose square vanishes beside 1), 16 ≤ s < 2^500
     // (overflowed ratios and NaN fail this), |n| ≥ 2^-460, or 2^-900 for s < 2^60
     // (the weights of values that small are the linear ones, s = 16), or a zero
-    // stencil, and no denominator beyond recip_sq
+    // stencil
     const unsigned hx = max(hi_bits(x0), max(hi_bits(x1), hi_bits(x2)));
     const unsigned hn = hi_bits(n) & 0x7fffffffu;
     const unsigned nlo = hi_bits(s) < ((1023u + 60u) << 20) ? (1023u - 900u) << 20 : 0x23300000u;
     const bool zero = (((hi_bits(Q0) | hi_bits(Q1) | hi_bits(Q2)) << 1) |
                        (unsigned)(__double2loint(Q0) | __double2loint(Q1) | __double2loint(Q2))) == 0u;
-    const unsigned lo = max(max(lo_bits(x0), lo_bits(s)), max(lo_bits(x1), lo_bits(x2)));
-    bad = bad || !sq_in(lo) || hx >= 0x5f300000u || hi_bits(s) >= 0x5f300000u || !(hn - nlo < 0x60000000u - nlo || zero);
+    bad = bad || hx >= 0x5f300000u || hi_bits(s) >= 0x5f300000u || !(hn - nlo < 0x60000000u - nlo || zero);
     return quot_rn(n, recip_sq(8.0 * s));
 }
 __device__ __forceinline__ void weno5z_pair_rn(const double* v, double& left, double& right, bool& bad) {
